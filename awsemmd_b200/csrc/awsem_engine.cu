@@ -305,6 +305,7 @@ template <typename R> class Engine : public EngineBase {
     // extent (on a serving handle the used prefix, not the whole capacity)
     a.fm.groups = std::min(fm_groups, (n_run() + 31) / 32);
     a.fm.dsplit = fm_dsplit;
+    a.fm.psplit = fm_psplit(fm_groups);
     a.fm.wait_limit = fm_wait_limit;
     a.fm.hold_tx = (hold_waits & 1) ? 16u : 0u;
     a.tb_data = reinterpret_cast<const double2 *>(tb_data.p);
@@ -1038,11 +1039,12 @@ template <typename R> class Engine : public EngineBase {
   }
 
   // one MD step (evaluation, Langevin, velocity Verlet) as one cooperative launch
-  void launch_step_persistent(const dev::StepArgs<R> &a)
+  void launch_step_persistent(dev::StepArgs<R> a)
   {
+    a.fm.psplit = 1;  // its warps take units one by one
     const bool fm = fm_on(a);
     dev::PersistArgs q{d_integ.p, g1.p, g2.p, ftot.p, x.p, gbar.p, n_run(), ps_stream,
-                       fm ? ps_ring_warps() : 0, fm ? std::min(fm_groups, (n_run() + 31) / 32) * fm_dsplit : 0,
+                       fm ? ps_ring_warps() : 0, fm ? fm_units() : 0,
                        (a.groups & dev::G_FIX) && (in.ff.p.terms & T_FM_TABLE) ? 1 : 0,
                        (a.groups & dev::G_FIX) && (in.ff.p.terms & T_AMHGO) ? 1 : 0,
                        (a.groups & dev::G_FIX) && (in.ff.p.terms & (T_SSB | T_DH | T_CONTREST)) ? 1 : 0,
@@ -1344,6 +1346,7 @@ template <typename R> class Engine : public EngineBase {
     v.min_sep = in.ff.p.fm_min_sep;
     v.groups = fm_groups;
     v.dsplit = fm_dsplit;
+    v.psplit = fm_psplit(fm_groups);
     v.n_res = n();
     v.is_double = sizeof(R) == sizeof(double);
     v.sigma_sq = in.ff.p.fm_sigma_sq;
@@ -1367,6 +1370,7 @@ template <typename R> class Engine : public EngineBase {
           len = std::max(len, fm.row_start[row + 1] - fm.row_start[row]);
         }
         len += len & 1;  // even: the kernels take a row's records in pairs
+        fm_rowmax = std::max(fm_rowmax, len);
         soff[(size_t) g * nd + d] = (int) stripes;
         slen[(size_t) g * nd + d] = len;
         stripes += len;
@@ -1395,15 +1399,29 @@ template <typename R> class Engine : public EngineBase {
     int sms = 148;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     fm_dsplit = std::max(1, std::min(std::max(nd, 1), (16 * sms + fm_groups - 1) / std::max(fm_groups, 1)));
+    // FP64 rows are long enough to be units of their own at every size, and
+    // evenly sized units end together
+    if (sizeof(R) == 8) fm_dsplit = std::max(nd, 1);
     CK(cudaStreamSynchronize(s0));  // host vectors go out of scope
   }
+
+  // FP64 with one separation a unit and rows of at most four pieces: a block of four warps shares a unit's row
+  // (awsem_fragmem.cuh) until such blocks fill the multiprocessors four times over (100 residues: 46 -> 11 us; at
+  // 17,000 residues, 3,240 units, a warp a unit is the faster by 5%)
+  int fm_rowmax = 0;  // stripes of the longest row
+  int fm_psplit(int groups) const
+  {
+    if (sizeof(R) == 4 || server || fm_dsplit != in.ff.p.fm_nd || fm_rowmax > dev::kFmPiece * dev::kFmBlockPieces) return 1;
+    return groups * fm_dsplit <= 4 * sms_ ? dev::kFmBlockPieces : 1;
+  }
+  int fm_units() const { return std::min(fm_groups, (n_run() + 31) / 32) * fm_dsplit; }
 
   // one warp per fragment-memory work unit, or a smaller persistent grid
   // (fm_grid blocks) whose warps loop over the units
   int fm_grid = 0;
   int fm_blocks() const
   {
-    const int all = (((n_run() + 31) / 32) * fm_dsplit * 32 + 127) / 128;
+    const int all = fm_psplit(fm_groups) > 1 ? fm_units() : (fm_units() * 32 + 127) / 128;
     return fm_grid > 0 ? std::min(all, fm_grid) : all;
   }
   // dynamic shared memory of a fragment-memory block (4 warps)

@@ -24,6 +24,15 @@
 // the accumulator of j with integer atomics; i's forces are summed in
 // registers over the chunk first.  Everything is order independent, so a
 // residue's result does not depend on its group mates or on the chunking.
+//
+// FP64 rows are summed in pieces of kFmPiece records, a piece's sums from zero
+// and added to the row's in order, so that the warps of a block can take the
+// pieces of one row and give the bits of one warp alone.  A record is four
+// FP64 exponentials (about 0.35 us for a warp that has its scheduler to
+// itself): on one chain of 100 residues the 24 (group, separation) units took
+// 46 us, the longest row's 120 records in series, while most of the chip was
+// idle.  FP32 rows keep two running sums (pieces would round differently) and
+// take 15 us on 2,000 residues.
 #pragma once
 
 #include "awsem_device.cuh"
@@ -40,6 +49,8 @@ template <typename R> struct FMSlices {
   int nd, min_sep;  // separations min_sep .. min_sep + nd - 1
   int groups;       // G = ceil(n_res / 32)
   int dsplit;       // separation chunks per group (warps per group)
+  int psplit;       // warps per unit: 4 (FP64, one separation a chunk, rows of at most 4 pieces: a block
+                    // takes a unit, a warp each piece of its row) or 1
   long long wait_limit;  // SM clock cycles a warp waits for one stage's copies before it gives up
   unsigned hold_tx;      // bytes each stage expects beyond its copies: 0, or (tests of the give-up
                          // path) 16, which never arrive, so every stage wait runs out
@@ -68,16 +79,64 @@ __device__ __forceinline__ void red_add3(unsigned long long *p, const long long 
 // Per-record arithmetic, shared by both load paths (so they agree bit for
 // bit).  The Gaussian of a row with variance s^2 is exp(-dr^2 / (2 s^2)):
 // FP32 evaluates it as 2^(k2 dr^2) with k2 = -log2(e) / (2 s^2) on the ex2
-// unit, FP64 as exp(k2 dr^2) with k2 = -1 / (2 s^2).
+// unit, FP64 as e^x with z = 32 x / ln2 = k2 dr^2.
 __device__ __forceinline__ float fm_gauss(float x)
 {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ double fm_gauss(double x) { return exp(x); }
+// FP64 Gaussians: e^x for x <= 0 by the table method of P. T. P. Tang ("Table-
+// driven implementation of the exponential function in IEEE floating-point
+// arithmetic", ACM TOMS 15 (1989)) in units of ln2 / 32: z = 32 x / ln2 = 32 m
+// + j + f with |f| <= 1/2, e^x = 2^m 2^(j/32) (1 + p(f)), p the Taylor
+// polynomial of 2^(f/32) - 1 to f^6 (remainder below 4e-18).  The row's factor
+// carries the 32 / ln2, so z - (32 m + j) is exact.  Lane j of the warp holds
+// 2^(j/32), read by a shuffle.  No branches and no calls: the exponentials of
+// a record pair are formed side by side.  Arguments below -708 (the padding's
+// -1e59 among them) give 0.  Every lane of the warp takes part.
+__device__ const double kExp2Of32nds[32] = {
+    0x1.0000000000000p+0, 0x1.059b0d3158574p+0, 0x1.0b5586cf9890fp+0, 0x1.11301d0125b51p+0,
+    0x1.172b83c7d517bp+0, 0x1.1d4873168b9aap+0, 0x1.2387a6e756238p+0, 0x1.29e9df51fdee1p+0,
+    0x1.306fe0a31b715p+0, 0x1.371a7373aa9cbp+0, 0x1.3dea64c123422p+0, 0x1.44e086061892dp+0,
+    0x1.4bfdad5362a27p+0, 0x1.5342b569d4f82p+0, 0x1.5ab07dd485429p+0, 0x1.6247eb03a5585p+0,
+    0x1.6a09e667f3bcdp+0, 0x1.71f75e8ec5f74p+0, 0x1.7a11473eb0187p+0, 0x1.82589994cce13p+0,
+    0x1.8ace5422aa0dbp+0, 0x1.93737b0cdc5e5p+0, 0x1.9c49182a3f090p+0, 0x1.a5503b23e255dp+0,
+    0x1.ae89f995ad3adp+0, 0x1.b7f76f2fb5e47p+0, 0x1.c199bdd85529cp+0, 0x1.cb720dcef9069p+0,
+    0x1.d5818dcfba487p+0, 0x1.dfc97337b9b5fp+0, 0x1.ea4afa2a490dap+0, 0x1.f50765b6e4540p+0,
+};
+template <typename R> struct GaussTable {};
+template <> struct GaussTable<double> {
+  double t = kExp2Of32nds[threadIdx.x & 31];
+};
+template <int N> __device__ __forceinline__ void fm_gauss(const double (&z)[N], const GaussTable<double> &tab, double (&g)[N])
+{
+  const double magic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the nearest integer
+  double y[N], f[N], q[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) y[k] = __dadd_rn(z[k], magic);
+#pragma unroll
+  for (int k = 0; k < N; k++) f[k] = __dsub_rn(z[k], __dsub_rn(y[k], magic));
+#pragma unroll
+  for (int k = 0; k < N; k++) q[k] = __fma_rn(f[k], 0x1.430912f86c787p-43, 0x1.5d87fe78a6731p-35);
+#pragma unroll
+  for (int k = 0; k < N; k++) q[k] = __fma_rn(f[k], q[k], 0x1.3b2ab6fba4e77p-27);
+#pragma unroll
+  for (int k = 0; k < N; k++) q[k] = __fma_rn(f[k], q[k], 0x1.c6b08d704a0c0p-20);
+#pragma unroll
+  for (int k = 0; k < N; k++) q[k] = __fma_rn(f[k], q[k], 0x1.ebfbdff82c58fp-13);
+#pragma unroll
+  for (int k = 0; k < N; k++) q[k] = __dmul_rn(f[k], __fma_rn(f[k], q[k], 0x1.62e42fefa39efp-6));
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const int n = __double2loint(y[k]);
+    const double t = __shfl_sync(0xffffffffu, tab.t, n & 31);
+    const double s = __hiloint2double(__double2hiint(t) + ((n >> 5) << 20), __double2loint(t));
+    g[k] = z[k] < -708.0 * 0x1.71547652b82fep+5 ? 0.0 : __fma_rn(s, q[k], s);
+  }
+}
 __device__ __forceinline__ float fm_k2(float s2) { return -1.4426950408889634f / (2.f * s2); }
-__device__ __forceinline__ double fm_k2(double s2) { return -1.0 / (2.0 * s2); }
+__device__ __forceinline__ double fm_k2(double s2) { return -0x1.71547652b82fep+5 / (2.0 * s2); }  // 32 / ln2
 
 // One record's four Gaussians g_k (times the record's coefficient when the
 // coefficients are not uniform): es += sum g_k, fs_k += g_k dr_k.  The row's
@@ -115,7 +174,7 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
 }
 
 template <bool COEF, typename R>
-__device__ __forceinline__ void fm_record(const R rec[4], R cc, const R r[4], R k2, R &es, R fs[4])
+__device__ __forceinline__ void fm_record(const GaussTable<R> &tab, const R rec[4], R cc, const R r[4], R k2, R &es, R fs[4])
 {
   if constexpr (sizeof(R) == 4) {
     // atom pairs (0, 1) and (2, 3) as f32x2 pairs: the same operations in
@@ -133,19 +192,173 @@ __device__ __forceinline__ void fm_record(const R rec[4], R cc, const R r[4], R 
       f2_unpack(f2_fma(f2_pack(g0, g1), dr, f2_pack(fs[h], fs[h + 1])), fs[h], fs[h + 1]);
     }
   } else {
+    double dr[4], z[4], g[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) dr[k] = r[k] - rec[k], z[k] = dr[k] * dr[k] * k2;
+    fm_gauss(z, tab, g);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const R dr = r[k] - rec[k];
-      R g = fm_gauss(dr * dr * k2);
-      if (COEF) g = g * cc;
-      es = es + g;
-      fs[k] = madd(g, dr, fs[k]);
+      if (COEF) g[k] = g[k] * cc;
+      es = es + g[k];
+      fs[k] = madd(g[k], dr[k], fs[k]);
     }
   }
 }
 
-// Work unit w (group g, chunk c of its separations) of the fragment-memory
-// term, records loaded into registers.  `pos(r, b)` returns the FP64
+// Records of an FP64 piece (a multiple of the copy stages' stripes); FP32 rows are one piece.
+constexpr int kFmPiece = 32, kFmBlockPieces = 4;
+template <typename R> __host__ __device__ constexpr int fm_piece() { return sizeof(R) == 8 ? kFmPiece : 1 << 30; }
+
+// Work unit w: chunk c (separations d0 <= d < d1) of group g; the stripes
+// [lo, hi) of its row when a block shares it, whole rows otherwise.
+struct FMUnit {
+  int g, d0, d1, lo, hi;
+};
+template <typename R> __device__ __forceinline__ FMUnit fm_unit(int w, const FMSlices<R> &t)
+{
+  const int g = w / t.dsplit, c = w - g * t.dsplit;
+  FMUnit q{g, c * t.nd / t.dsplit, (c + 1) * t.nd / t.dsplit, 0, 1 << 30};
+  if (sizeof(R) == 8 && t.psplit > 1) {
+    q.lo = kFmPiece * (threadIdx.x >> 5);
+    q.hi = q.lo + kFmPiece;
+  }
+  return q;
+}
+
+// Geometry of row (i, j): the four atom-pair differences and distances
+template <typename R, class Pos>
+__device__ __forceinline__ void fm_row_geometry(const Pos &pos, int i, int j, V3<R> dv[4], R r[4])
+{
+  const V3<double> ca_i = pos(i, 0), cb_i = pos(i, 1), ca_j = pos(j, 0), cb_j = pos(j, 1);
+  dv[0] = diff<R>(ca_i, ca_j);
+  dv[1] = diff<R>(ca_i, cb_j);
+  dv[2] = diff<R>(cb_i, ca_j);
+  dv[3] = diff<R>(cb_i, cb_j);
+#pragma unroll
+  for (int k = 0; k < 4; k++) r[k] = m_sqrt(norm2(dv[k]));
+}
+
+// Sums of the rows of one unit: the running sums of the current piece, in FP64
+// the row's, and in FP32 the unit's forces on residue i in fixed point.  FP64
+// rows add their forces on i to memory as they end, from differences formed
+// again there: what the record loop holds then fits 12 warps per
+// multiprocessor without spills (all in registers: 242, 8 warps).
+template <typename R> struct FMSums {
+  R es = 0, fs[4] = {0, 0, 0, 0}, es1 = 0, fs1[4] = {0, 0, 0, 0};  // even and odd records
+  R et = 0, ft[4] = {0, 0, 0, 0};                                  // FP64: the row's pieces so far
+  long long fca[3] = {0, 0, 0}, fcb[3] = {0, 0, 0};
+  double e = 0.0;
+
+  // a piece ends
+  __device__ __forceinline__ void end_piece()
+  {
+    if constexpr (sizeof(R) == 8) {
+      et = et + (es + es1);
+#pragma unroll
+      for (int k = 0; k < 4; k++) ft[k] = ft[k] + (fs[k] + fs1[k]);
+    } else {
+      et = es + es1;
+#pragma unroll
+      for (int k = 0; k < 4; k++) ft[k] = fs[k] + fs1[k];
+    }
+    es = es1 = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) fs[k] = fs1[k] = 0;
+  }
+  // the row (i, j) ends: its sums to fixed point
+  template <class Pos>
+  __device__ __forceinline__ void end_row(R scale, R s2, const R r[4], const V3<R> dv[4], const Pos &pos, int ii,
+                                          bool live, int j, unsigned long long *facc)
+  {
+    e += (double) (scale * et);
+    long long fja[3] = {0, 0, 0}, fjb[3] = {0, 0, 0};
+    if constexpr (sizeof(R) == 8) {
+      V3<R> dp[4];
+      R rp[4];
+      fm_row_geometry(pos, ii, j, dp, rp);
+      split(scale, s2, rp, dp, fca, fcb, fja, fjb);
+      if (live) {
+        red_add3(facc + (size_t) 9 * ii, fca);
+        red_add3(facc + (size_t) 9 * ii + 3, fcb);
+      }
+#pragma unroll
+      for (int q = 0; q < 3; q++) fca[q] = fcb[q] = 0;
+    } else {
+      split(scale, s2, r, dv, fca, fcb, fja, fjb);
+    }
+    red_add3(facc + (size_t) 9 * j, fja);
+    red_add3(facc + (size_t) 9 * j + 3, fjb);
+    et = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) ft[k] = 0;
+  }
+  // atom pair k acts on CA(i) (k < 2) or CB(i), and on CA(j) (k even) or CB(j)
+  __device__ __forceinline__ void split(R scale, R s2, const R r[4], const V3<R> dv[4], long long ga[3], long long gb[3],
+                                        long long ha[3], long long hb[3]) const
+  {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const R fc = ft[k] != R(0) ? (scale * ft[k]) / (s2 * r[k]) : R(0);
+      const long long v[3] = {fix_force((double) (fc * dv[k].x)), fix_force((double) (fc * dv[k].y)),
+                              fix_force((double) (fc * dv[k].z))};
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        if (k < 2)
+          ga[q] += v[q];
+        else
+          gb[q] += v[q];
+        if (k & 1)
+          hb[q] -= v[q];
+        else
+          ha[q] -= v[q];
+      }
+    }
+  }
+  // the unit ends
+  __device__ __forceinline__ void end_unit(bool live, int i, unsigned long long *facc, unsigned long long *e_acc,
+                                           int e_stride)
+  {
+    if (sizeof(R) == 4 && live) {
+      red_add3(facc + (size_t) 9 * i, fca);
+      red_add3(facc + (size_t) 9 * i + 3, fcb);
+    }
+    long long en = live ? fix_force(e) : 0;
+    if (e_stride) {
+      if (en) atomicAdd(e_acc + (size_t) i * e_stride, (unsigned long long) en);
+    } else {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) en += __shfl_xor_sync(0xffffffffu, en, o);
+      if ((threadIdx.x & 31) == 0 && en) atomicAdd(e_acc, (unsigned long long) en);
+    }
+  }
+};
+
+// The pieces of a block's row meet (psplit > 1; every thread of the block
+// takes part): warp p has piece p's sums (zero where the row has none), and
+// warp 0 adds them in order, as one warp alone does.  Returns whether this
+// warp now holds the row.
+__device__ __forceinline__ bool fm_join_pieces(FMSums<double> &s)
+{
+  __shared__ double xch[kFmBlockPieces - 1][5][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp) {
+    xch[warp - 1][4][lane] = s.et;
+#pragma unroll
+    for (int k = 0; k < 4; k++) xch[warp - 1][k][lane] = s.ft[k];
+  }
+  __syncthreads();
+  if (warp) return false;
+#pragma unroll
+  for (int p = 0; p < kFmBlockPieces - 1; p++) {
+    s.et = s.et + xch[p][4][lane];
+#pragma unroll
+    for (int k = 0; k < 4; k++) s.ft[k] = s.ft[k] + xch[p][k][lane];
+  }
+  return true;
+}
+__device__ __forceinline__ bool fm_join_pieces(FMSums<float> &) { return true; }
+
+// Work unit w of the fragment-memory term, records loaded into registers.  `pos(r, b)` returns the FP64
 // position of residue r's CA (b = 0) or CB (b = 1); forces go to `facc`
 // ([atom][3], atom = 3 r + b, fixed point).  Energies are added in fixed
 // point to e_acc[i * e_stride] (per residue with e_stride = 1; one total
@@ -157,77 +370,42 @@ __device__ __forceinline__ void fragmem_unit_reg_t(int w, const FMSlices<R> &t, 
                                                    unsigned long long *e_acc, int e_stride)
 {
   const int lane = threadIdx.x & 31;
-  const int g = w / t.dsplit, c = w - g * t.dsplit;
-  const int d0 = c * t.nd / t.dsplit, d1 = (c + 1) * t.nd / t.dsplit;
-  const int i = g * 32 + lane;
+  const FMUnit u = fm_unit(w, t);
+  const int i = u.g * 32 + lane;
   const bool live = i < n;
   const int ii = live ? i : n - 1;
-  const V3<double> ca_i = pos(ii, 0), cb_i = pos(ii, 1);
-  long long fca[3] = {0, 0, 0}, fcb[3] = {0, 0, 0};
-  double e = 0.0;
   const R scale = COEF ? R(-1) : -R(t.uniform);
-  for (int d = d0; d < d1; d++) {
-    const int blk = g * t.nd + d;
-    const int len = t.slen[blk];
-    if (len == 0) continue;
+  FMSums<R> sum;
+  const GaussTable<R> tab;
+  for (int d = u.d0; d < u.d1; d++) {
+    const int blk = u.g * t.nd + d;
+    const int hi = min(u.hi, t.slen[blk]);
+    if (t.slen[blk] == 0) continue;
     const size_t base = (size_t) t.soff[blk] * 32 + lane;
     // rows past the end carry padding only; any valid partner index will do
     const int j = min(ii + t.min_sep + d, n - 1);
-    const V3<double> ca_j = pos(j, 0), cb_j = pos(j, 1);
-    const V3<R> dv[4] = {diff<R>(ca_i, ca_j), diff<R>(ca_i, cb_j), diff<R>(cb_i, ca_j), diff<R>(cb_i, cb_j)};
+    V3<R> dv[4];
     R r[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) r[k] = m_sqrt(norm2(dv[k]));
+    fm_row_geometry(pos, ii, j, dv, r);
     const R s2 = R(sig[t.min_sep + d]);
     const R k2 = fm_k2(s2);
-    R es = 0, fs[4] = {0, 0, 0, 0}, es1 = 0, fs1[4] = {0, 0, 0, 0};
+    for (int p0 = u.lo; p0 < hi; p0 += fm_piece<R>()) {
+      const int p1 = min(hi - p0, fm_piece<R>()) + p0;
 #pragma unroll 2
-    for (int m = 0; m < len; m += 2) {  // len is even
-      const size_t at = base + (size_t) m * 32;
-      R rec[4], rec1[4];
-      load_record(t.rf, at, rec);
-      load_record(t.rf, at + 32, rec1);
-      fm_record<COEF>(rec, COEF ? t.coef[at] : R(1), r, k2, es, fs);
-      fm_record<COEF>(rec1, COEF ? t.coef[at + 32] : R(1), r, k2, es1, fs1);
-    }
-    es = es + es1;
-#pragma unroll
-    for (int k = 0; k < 4; k++) fs[k] = fs[k] + fs1[k];
-    e += (double) (scale * es);
-    // atom pair k acts on CA(i) (k < 2) or CB(i), and on CA(j) (k even) or CB(j)
-    long long fja[3] = {0, 0, 0}, fjb[3] = {0, 0, 0};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const R fc = fs[k] != R(0) ? (scale * fs[k]) / (s2 * r[k]) : R(0);
-      const long long v[3] = {fix_force((double) (fc * dv[k].x)), fix_force((double) (fc * dv[k].y)),
-                              fix_force((double) (fc * dv[k].z))};
-#pragma unroll
-      for (int q = 0; q < 3; q++) {
-        if (k < 2)
-          fca[q] += v[q];
-        else
-          fcb[q] += v[q];
-        if (k & 1)
-          fjb[q] -= v[q];
-        else
-          fja[q] -= v[q];
+      for (int m = p0; m < p1; m += 2) {  // block lengths and pieces are even
+        const size_t at = base + (size_t) m * 32;
+        R rec[4], rec1[4];
+        load_record(t.rf, at, rec);
+        load_record(t.rf, at + 32, rec1);
+        fm_record<COEF>(tab, rec, COEF ? t.coef[at] : R(1), r, k2, sum.es, sum.fs);
+        fm_record<COEF>(tab, rec1, COEF ? t.coef[at + 32] : R(1), r, k2, sum.es1, sum.fs1);
       }
+      sum.end_piece();
     }
-    red_add3(facc + (size_t) 9 * j, fja);
-    red_add3(facc + (size_t) 9 * j + 3, fjb);
+    if (sizeof(R) == 8 && t.psplit > 1 && !fm_join_pieces(sum)) return;
+    sum.end_row(scale, s2, r, dv, pos, ii, live, j, facc);
   }
-  if (live) {
-    red_add3(facc + (size_t) 9 * i, fca);
-    red_add3(facc + (size_t) 9 * i + 3, fcb);
-  }
-  long long ef = live ? fix_force(e) : 0;
-  if (e_stride) {
-    if (ef) atomicAdd(e_acc + (size_t) i * e_stride, (unsigned long long) ef);
-  } else {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ef += __shfl_xor_sync(0xffffffffu, ef, o);
-    if (lane == 0 && ef) atomicAdd(e_acc, (unsigned long long) ef);
-  }
+  sum.end_unit(live, i, facc, e_acc, e_stride);
 }
 
 template <typename R, class Pos>
@@ -240,31 +418,118 @@ __device__ __forceinline__ void fragmem_unit_reg(int w, const FMSlices<R> &t, co
     fragmem_unit_reg_t<false>(w, t, sig, n, pos, facc, e_acc, e_stride);
 }
 
-// one warp per work unit
+// FP32 rows by two warps: warp h (0, 1) of the pair takes a row's even or odd
+// records, one of the row's two sets of sums, so the sums are a single warp's
+// bit for bit.  Eight records are loaded ahead of their arithmetic.  The odd
+// warp hands its sums over in shared memory (xch: two buffers of 5 x 32
+// floats, used in turn, so one barrier a row suffices; `bar` is the pair's
+// named barrier).  For callers with a warp per unit and no copy ring: on 8,000
+// residues with weighted memories (66 MB) a single warp's 120 records in
+// series, four loads in flight, held the call at 36 us.
+template <bool COEF, class Pos>
+__device__ __forceinline__ void fragmem_unit_pair(int w, int h, const FMSlices<float> &t, const double *sig, int n,
+                                                  const Pos &pos, unsigned long long *facc, unsigned long long *e_acc,
+                                                  int e_stride, float *xch, int bar)
+{
+  constexpr int kAhead = 8;
+  const int lane = threadIdx.x & 31;
+  const FMUnit u = fm_unit(w, t);
+  const int i = u.g * 32 + lane;
+  const bool live = i < n;
+  const int ii = live ? i : n - 1;
+  const float scale = COEF ? -1.f : -(float) t.uniform;
+  FMSums<float> sum;
+  const GaussTable<float> tab;
+  int turn = 0;
+  for (int d = u.d0; d < u.d1; d++) {
+    const int blk = u.g * t.nd + d, len = t.slen[blk];
+    if (len == 0) continue;
+    const size_t base = ((size_t) t.soff[blk] + h) * 32 + lane;
+    const int j = min(ii + t.min_sep + d, n - 1), half = len / 2;  // len is even
+    float rec[kAhead][4], cf[kAhead];
+    auto load = [&](int k, int m) {
+      const size_t at = base + (size_t) m * 64;
+      load_record(t.rf, at, rec[k]);
+      cf[k] = COEF ? t.coef[at] : 1.f;
+    };
+#pragma unroll
+    for (int k = 0; k < kAhead; k++)
+      if (k < half) load(k, k);
+    V3<float> dv[4];
+    float r[4];
+    fm_row_geometry(pos, ii, j, dv, r);
+    const float s2 = (float) sig[t.min_sep + d], k2 = fm_k2(s2);
+    for (int m0 = 0; m0 < half; m0 += kAhead) {
+#pragma unroll
+      for (int k = 0; k < kAhead; k++) {
+        if (m0 + k < half) fm_record<COEF>(tab, rec[k], cf[k], r, k2, sum.es, sum.fs);
+        if (m0 + k + kAhead < half) load(k, m0 + k + kAhead);
+      }
+    }
+    float *buf = xch + turn * 160 + lane;
+    turn ^= 1;
+    if (h) {
+      buf[0] = sum.es;
+#pragma unroll
+      for (int k = 0; k < 4; k++) buf[32 * (k + 1)] = sum.fs[k];
+    }
+    asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+    if (!h) {
+      sum.es1 = buf[0];
+#pragma unroll
+      for (int k = 0; k < 4; k++) sum.fs1[k] = buf[32 * (k + 1)];
+      sum.end_piece();
+      sum.end_row(scale, s2, r, dv, pos, ii, live, j, facc);
+    } else {
+      sum.es = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; k++) sum.fs[k] = 0.f;
+    }
+  }
+  if (!h) sum.end_unit(live, i, facc, e_acc, e_stride);
+}
+
+// A launch with one warp (FP64; a block where it shares a row) or one
+// warp pair (FP32) per work unit, 128 threads a block
+template <typename R> constexpr int kFmUnitWarps = sizeof(R) == 4 ? 2 : 1;
 template <typename R, class Pos>
 __device__ __forceinline__ void fragmem_warp(const FMSlices<R> &t, const double *sig, int n, const Pos &pos,
                                              unsigned long long *facc, unsigned long long *e_acc, int e_stride)
 {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w < t.groups * t.dsplit) fragmem_unit_reg(w, t, sig, n, pos, facc, e_acc, e_stride);
+  if constexpr (sizeof(R) == 4) {
+    __shared__ float xch[2][320];
+    const int pair = (threadIdx.x >> 6) & 1;
+    if (w / 2 >= t.groups * t.dsplit) return;  // both warps of the pair
+    if (t.coef)
+      fragmem_unit_pair<true>(w / 2, w & 1, t, sig, n, pos, facc, e_acc, e_stride, xch[pair], 1 + pair);
+    else
+      fragmem_unit_pair<false>(w / 2, w & 1, t, sig, n, pos, facc, e_acc, e_stride, xch[pair], 1 + pair);
+  } else {
+    const int u = t.psplit > 1 ? (int) blockIdx.x : w;
+    if (u < t.groups * t.dsplit) fragmem_unit_reg(u, t, sig, n, pos, facc, e_acc, e_stride);
+  }
 }
-
 
 // ---------------------------------------------------------------------------
 // Bulk-copy pipeline.  A group's blocks are contiguous stripes, so a warp's
 // whole share is one contiguous run of stripes: lane 0 streams it into a
-// ring of kFmStages shared-memory stages of kFmStripes stripes with 1-D bulk
+// ring of kFmStages shared-memory stages of kFmStripes<R> stripes with 1-D bulk
 // copies (cp.async.bulk, the TMA engine) completing on one mbarrier per
 // stage, and the 32 lanes read their records from shared memory.  Up to
 // kFmStages stages are in flight per warp with no register cost, which is
 // what the register-load version lacks at full size.  Per lane the records
 // are consumed in the same order, so the sums equal the register version's
 // bit for bit.
-constexpr int kFmStages = 3, kFmStripes = 8;
+// A stage is 4 KiB of distances in both forms: eight FP32 stripes (bandwidth
+// bound: 3 x 4 KiB in flight a warp) or four FP64 ones (arithmetic bound; with
+// eight, 25 KiB a warp left room for 8 warps per SM).
+constexpr int kFmStages = 3;
+template <typename R> constexpr int kFmStripes = sizeof(R) == 4 ? 8 : 4;
 
 template <typename R> __host__ __device__ constexpr int fm_stage_bytes(bool coef)
 {
-  return kFmStripes * 32 * (int) sizeof(R) * (coef ? 5 : 4);
+  return kFmStripes<R> * 32 * (int) sizeof(R) * (coef ? 5 : 4);
 }
 // shared memory of one warp: 128 bytes of mbarriers, then the stages
 template <typename R> __host__ __device__ constexpr int fm_warp_smem(bool coef)
@@ -333,8 +598,8 @@ __device__ __forceinline__ bool fragmem_unit_bulk_t(int w, const FMSlices<R> &t,
                                                     unsigned char *wsm, unsigned &kbase)
 {
   const int lane = threadIdx.x & 31;
-  const int g = w / t.dsplit, c = w - g * t.dsplit;
-  const int d0 = c * t.nd / t.dsplit, d1 = (c + 1) * t.nd / t.dsplit;
+  const FMUnit u = fm_unit(w, t);
+  const int g = u.g, d1 = u.d1;
   const int i = g * 32 + lane;
   const bool live = i < n;
   const int ii = live ? i : n - 1;
@@ -343,78 +608,48 @@ __device__ __forceinline__ bool fragmem_unit_bulk_t(int w, const FMSlices<R> &t,
   const uint32_t bars = smem_addr(wsm), data = bars + 128;
   // the warp's run of stripes: its non-empty blocks, contiguous from the first
   int first = -1, total = 0;
-  for (int dd = d0; dd < d1; dd++) {
-    const int len = t.slen[g * t.nd + dd];
-    if (len > 0 && first < 0) first = t.soff[g * t.nd + dd];
+  for (int dd = u.d0; dd < d1; dd++) {
+    const int len = min(u.hi, t.slen[g * t.nd + dd]) - u.lo;
+    if (len <= 0) continue;
+    if (first < 0) first = t.soff[g * t.nd + dd] + u.lo;
     total += len;
   }
-  if (total <= 0) return true;
-  const int last = first + total, nchunks = (total + kFmStripes - 1) / kFmStripes;
+  FMSums<R> sum;
+  if (total <= 0) {
+    // a block's warp without a piece still joins the others
+    if (sizeof(R) == 8 && t.psplit > 1 && t.slen[g * t.nd + u.d0] > 0) fm_join_pieces(sum);
+    return true;
+  }
+  const int last = first + total, nchunks = (total + kFmStripes<R> - 1) / kFmStripes<R>;
   auto issue = [&](int k) {  // lane 0: chunk k into stage (kbase + k) % kFmStages
-    const int st = (kbase + k) % kFmStages, s0 = first + k * kFmStripes, ns = min(kFmStripes, last - s0);
+    const int st = (kbase + k) % kFmStages, s0 = first + k * kFmStripes<R>, ns = min(kFmStripes<R>, last - s0);
     const uint32_t bar = bars + 8 * st, dst = data + st * stage_bytes;
     const uint32_t rb = ns * 32 * 4 * sizeof(R), cb = coef ? ns * 32 * sizeof(R) : 0;
     // the stage was last read through the generic proxy: order that before the async-proxy write
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     mbar_expect(bar, rb + cb + t.hold_tx);
     bulk_load(dst, t.rf + (size_t) s0 * 32 * 4, rb, bar);
-    if (coef) bulk_load(dst + kFmStripes * 32 * 4 * sizeof(R), t.coef + (size_t) s0 * 32, cb, bar);
+    if (coef) bulk_load(dst + kFmStripes<R> * 32 * 4 * sizeof(R), t.coef + (size_t) s0 * 32, cb, bar);
   };
   if (lane == 0)
     for (int k = 0; k < kFmStages && k < nchunks; k++) issue(k);
 
-  const V3<double> ca_i = pos(ii, 0), cb_i = pos(ii, 1);
-  long long fca[3] = {0, 0, 0}, fcb[3] = {0, 0, 0};
-  double e = 0.0;
   const R scale = COEF ? R(-1) : -R(t.uniform);
-  // current row (block d): geometry and sums
-  int d = d0, blk_end = 0, j = 0;
+  const GaussTable<R> tab;
+  // current row (block d): geometry, its end and its current piece's end
+  int d = u.d0, row_end = 0, piece_end = 0, j = 0;
   V3<R> dv[4];
-  R r[4], s2 = 1, k2 = -1, es = 0, fs[4] = {0, 0, 0, 0}, es1 = 0, fs1[4] = {0, 0, 0, 0};
+  R r[4], s2 = 1, k2 = -1;
   auto begin_row = [&]() {  // d: the next non-empty block at or after d
     while (d < d1 && t.slen[g * t.nd + d] == 0) d++;
     if (d >= d1) return;
-    blk_end = t.soff[g * t.nd + d] - first + t.slen[g * t.nd + d];
+    const int row0 = t.soff[g * t.nd + d] + u.lo - first;
+    row_end = row0 + min(u.hi, t.slen[g * t.nd + d]) - u.lo;
+    piece_end = min(row_end - row0, fm_piece<R>()) + row0;
     j = min(ii + t.min_sep + d, n - 1);
-    const V3<double> ca_j = pos(j, 0), cb_j = pos(j, 1);
-    dv[0] = diff<R>(ca_i, ca_j);
-    dv[1] = diff<R>(ca_i, cb_j);
-    dv[2] = diff<R>(cb_i, ca_j);
-    dv[3] = diff<R>(cb_i, cb_j);
-#pragma unroll
-    for (int k = 0; k < 4; k++) r[k] = m_sqrt(norm2(dv[k]));
+    fm_row_geometry(pos, ii, j, dv, r);
     s2 = R(sig[t.min_sep + d]);
     k2 = fm_k2(s2);
-    es = es1 = 0;
-#pragma unroll
-    for (int k = 0; k < 4; k++) fs[k] = fs1[k] = 0;
-  };
-  auto end_row = [&]() {
-    es = es + es1;
-#pragma unroll
-    for (int k = 0; k < 4; k++) fs[k] = fs[k] + fs1[k];
-    e += (double) (scale * es);
-    long long fja[3] = {0, 0, 0}, fjb[3] = {0, 0, 0};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const R fc = fs[k] != R(0) ? (scale * fs[k]) / (s2 * r[k]) : R(0);
-      const long long v[3] = {fix_force((double) (fc * dv[k].x)), fix_force((double) (fc * dv[k].y)),
-                              fix_force((double) (fc * dv[k].z))};
-#pragma unroll
-      for (int q = 0; q < 3; q++) {
-        if (k < 2)
-          fca[q] += v[q];
-        else
-          fcb[q] += v[q];
-        if (k & 1)
-          fjb[q] -= v[q];
-        else
-          fja[q] -= v[q];
-      }
-    }
-    red_add3(facc + (size_t) 9 * j, fja);
-    red_add3(facc + (size_t) 9 * j + 3, fjb);
-    d++;
   };
   begin_row();
   bool ok = true;
@@ -429,24 +664,30 @@ __device__ __forceinline__ bool fragmem_unit_bulk_t(int w, const FMSlices<R> &t,
     }
     const unsigned char *sd = wsm + 128 + st * stage_bytes;
     const R *srf = reinterpret_cast<const R *>(sd);
-    const R *scf = reinterpret_cast<const R *>(sd + kFmStripes * 32 * 4 * sizeof(R));
-    const int s0 = k * kFmStripes, ns = min(kFmStripes, total - s0);
+    const R *scf = reinterpret_cast<const R *>(sd + kFmStripes<R> * 32 * 4 * sizeof(R));
+    const int s0 = k * kFmStripes<R>, ns = min(kFmStripes<R>, total - s0);
     for (int q = 0; q < ns;) {
-      while (s0 + q >= blk_end && d < d1) {  // rows end on stripe boundaries
-        end_row();
-        begin_row();
+      while (s0 + q >= piece_end && d < d1) {  // pieces and rows end on stripe boundaries
+        sum.end_piece();
+        if (sizeof(R) == 8 && piece_end < row_end) {  // FP32 rows are one piece
+          piece_end = min(row_end - piece_end, fm_piece<R>()) + piece_end;
+        } else {
+          sum.end_row(scale, s2, r, dv, pos, ii, live, j, facc);
+          d++;
+          begin_row();
+        }
       }
-      // the stripes of this chunk that belong to the current row (rows,
+      // the stripes of this chunk that belong to the current piece (pieces,
       // chunks and their ends fall on even stripes: records pair up as in
       // the register path)
-      const int run = max(q + 2, min(ns, blk_end - s0));
+      const int run = max(q + 2, min(ns, piece_end - s0));
 #pragma unroll(sizeof(R) == 4 ? 2 : 1)
       for (; q < run; q += 2) {
         R rec[4], rec1[4];
         load_record_shared(srf, q * 32 + lane, rec);
         load_record_shared(srf, (q + 1) * 32 + lane, rec1);
-        fm_record<COEF>(rec, COEF ? scf[q * 32 + lane] : R(1), r, k2, es, fs);
-        fm_record<COEF>(rec1, COEF ? scf[(q + 1) * 32 + lane] : R(1), r, k2, es1, fs1);
+        fm_record<COEF>(tab, rec, COEF ? scf[q * 32 + lane] : R(1), r, k2, sum.es, sum.fs);
+        fm_record<COEF>(tab, rec1, COEF ? scf[(q + 1) * 32 + lane] : R(1), r, k2, sum.es1, sum.fs1);
       }
     }
     __syncwarp();  // every lane has read the stage
@@ -457,22 +698,14 @@ __device__ __forceinline__ bool fragmem_unit_bulk_t(int w, const FMSlices<R> &t,
     if (lane == 0) atomicExch(timed_out, 1);
     for (int k = fail_k; k < nchunks && k < fail_k + kFmStages; k++)
       mbar_wait(bars + 8 * ((kbase + k) % kFmStages), ((kbase + k) / kFmStages) & 1, kFmWaitLimit / 8);
+    if (sizeof(R) == 8 && t.psplit > 1) fm_join_pieces(sum);  // the block's other warps wait there
     return false;
   }
   kbase += nchunks;
-  end_row();
-  if (live) {
-    red_add3(facc + (size_t) 9 * i, fca);
-    red_add3(facc + (size_t) 9 * i + 3, fcb);
-  }
-  long long ef = live ? fix_force(e) : 0;
-  if (e_stride) {
-    if (ef) atomicAdd(e_acc + (size_t) i * e_stride, (unsigned long long) ef);
-  } else {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ef += __shfl_xor_sync(0xffffffffu, ef, o);
-    if (lane == 0 && ef) atomicAdd(e_acc, (unsigned long long) ef);
-  }
+  sum.end_piece();
+  if (sizeof(R) == 8 && t.psplit > 1 && !fm_join_pieces(sum)) return true;
+  sum.end_row(scale, s2, r, dv, pos, ii, live, j, facc);
+  sum.end_unit(live, i, facc, e_acc, e_stride);
   return true;
 }
 
@@ -510,6 +743,17 @@ __device__ __forceinline__ void fragmem_warp_take(const FMSlices<R> &t, const do
   const int units = t.groups * t.dsplit, lane = threadIdx.x & 31;
   fragmem_ring_init(wsm);
   unsigned kbase = 0;
+  if (sizeof(R) == 8 && t.psplit > 1) {  // a block takes a unit (both barriers: its warps stay together, also when one's wait gave up)
+    __shared__ int s_u;
+    while (true) {
+      if (threadIdx.x == 0) s_u = atomicAdd(next, 1);
+      __syncthreads();
+      const int u = s_u;
+      if (u >= units) return;
+      const bool ok = fragmem_unit_bulk(u, t, sig, n, pos, facc, e_acc, e_stride, timed_out, wsm, kbase);
+      if (!__syncthreads_and(ok)) return;
+    }
+  }
   while (true) {
     int u = 0;
     if (lane == 0) u = atomicAdd(next, 1);
@@ -527,7 +771,7 @@ struct FMView {
   const int *soff, *slen;
   const void *rf, *coef;  // double (FP64 form) or float (mixed form) elements
   double uniform;
-  int nd, min_sep, groups, dsplit, n_res, is_double;
+  int nd, min_sep, groups, dsplit, psplit, n_res, is_double;
   const double *sigma_sq;  // host table [64]
 };
 

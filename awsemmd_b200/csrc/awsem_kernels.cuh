@@ -1339,8 +1339,9 @@ template <typename R> struct BeadPos {
   __device__ __forceinline__ V3<double> operator()(int r, int b) const { return bead(*s, r, b ? B_CB : B_CA); }
 };
 
+template <typename R> constexpr int kFmMinBlocks = sizeof(R) == 4 ? 4 : 3;
 // 128 threads, fm_warp_smem<R>(coef) bytes of dynamic shared memory per warp
-template <typename R> __global__ void __launch_bounds__(128) k_fragmem(StepArgs<R> a, FFParams p)
+template <typename R> __global__ void __launch_bounds__(128, kFmMinBlocks<R>) k_fragmem(StepArgs<R> a, FFParams p)
 {
   extern __shared__ __align__(128) unsigned char fm_smem[];
   const BeadPos<R> pos{&a.s};

@@ -130,6 +130,7 @@ template <typename R> dev::FMSlices<R> slices(const FMView &v)
   t.min_sep = v.min_sep;
   t.groups = v.groups;
   t.dsplit = v.dsplit;
+  t.psplit = v.psplit;
   t.wait_limit = dev::kFmWaitLimit;  // the register-load path used here has no waits
   t.hold_tx = 0;
   return t;
@@ -152,7 +153,8 @@ void fragmem_noalloc(int device, const FMView &v, const double *d_x, double *d_f
   int n3 = 3 * n_atoms, tb = 256;
   k_clear<<<(n3 + tb - 1) / tb, tb, 0, stream>>>(facc, n3);
   if (v.nd > 0) {
-    int blocks = (v.groups * v.dsplit * 32 + 127) / 128;
+    const int warps = v.is_double ? dev::kFmUnitWarps<double> : dev::kFmUnitWarps<float>;
+    int blocks = (v.groups * v.dsplit * v.psplit * warps * 32 + 127) / 128;
     if (v.is_double)
       k_fragmem<double><<<blocks, 128, 0, stream>>>(d_x, v.n_res, slices<double>(v), sig, facc);
     else
