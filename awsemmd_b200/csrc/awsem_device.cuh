@@ -379,18 +379,18 @@ __device__ void dihedral(const DevSys<R> &s, const FFParams &p, int i, int phi, 
 // cos(phi + phi0) and sin(phi + phi0) by the angle-sum identities from the
 // dihedral's own cosine and sine and the well's constant cos / sin phi0,
 // instead of an atan2 and four trigonometric calls per well.
-template <typename R> __device__ R rama_term(const DevSys<R> &s, const FFParams &p, int i)
+// The wells at (phi, psi) given as cosine and sine: the energy, and the
+// factors g0, g1 of the phi and psi slopes.
+template <typename R>
+__device__ __forceinline__ R rama_wells(const DevSys<R> &s, const FFParams &p, int i, R cf, R sf, R cs, R ss, R &g0, R &g1)
 {
-  R cf, sf, cs, ss;
-  V3<R> sphi[5], spsi[5];
-  dihedral(s, p, i, 1, cf, sf, sphi);
-  dihedral(s, p, i, 0, cs, ss, spsi);
   int j0 = 0, j1 = p.n_rama;
   if ((s.res_flags[i] & R_PRO) && (p.terms & T_RAMA_P)) {
     j0 = 6;
     j1 = 6 + p.n_rama_p;
   }
-  R E = 0, g0 = 0, g1 = 0;
+  R E = 0;
+  g0 = g1 = 0;
   for (int j = j0; j < j1; j++) {
     double aps = s.aps[(size_t) j * s.n_res + i];
     if (p.ssweight[j] && aps == 0.0) continue;
@@ -405,6 +405,15 @@ template <typename R> __device__ R rama_term(const DevSys<R> &s, const FFParams 
     g1 += f * sc * (ss * c1 + cs * s1);
     E += -V;
   }
+  return E;
+}
+template <typename R> __device__ R rama_term(const DevSys<R> &s, const FFParams &p, int i)
+{
+  R cf, sf, cs, ss, g0, g1;
+  V3<R> sphi[5], spsi[5];
+  dihedral(s, p, i, 1, cf, sf, sphi);
+  dihedral(s, p, i, 0, cs, ss, spsi);
+  const R E = rama_wells(s, p, i, cf, sf, cs, ss, g0, g1);
   if (g0 != R(0) || g1 != R(0)) {
     const int rr[5] = {i - 1, i, i + 1, i - 1, i};
     const int bb[5] = {B_CA, B_CA, B_CA, B_O, B_O};

@@ -164,7 +164,8 @@ template <typename R> class Engine : public EngineBase {
   cudaStream_t s0 = nullptr, s1 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaStream_t s2 = nullptr;  // the detection pass and the hydrogen-bond terms
-  cudaEvent_t ev_dens = nullptr, ev_join2 = nullptr;
+  cudaStream_t s3 = nullptr;  // the backbone terms
+  cudaEvent_t ev_dens = nullptr, ev_join2 = nullptr, ev_join3 = nullptr;
   DBuf<int> res_type, res_flags, res_chain, chain_start, chain_end, atom_tag, atom_type;
   DBuf<double> aps, tables, x, v, mass, g1, g2, ftot, work, e_res, energy;
   DBuf<double4> pos, cpos, cb_build;
@@ -229,9 +230,11 @@ template <typename R> class Engine : public EngineBase {
     if (ev_join) cudaEventDestroy(ev_join);
     if (ev_dens) cudaEventDestroy(ev_dens);
     if (ev_join2) cudaEventDestroy(ev_join2);
+    if (ev_join3) cudaEventDestroy(ev_join3);
     if (s0) cudaStreamDestroy(s0);
     if (s1) cudaStreamDestroy(s1);
     if (s2) cudaStreamDestroy(s2);
+    if (s3) cudaStreamDestroy(s3);
   }
 
   int n() const { return in.top.n_res; }
@@ -274,6 +277,7 @@ template <typename R> class Engine : public EngineBase {
     a.pairs = pairs.p;
     a.cpairs = cpairs.p;
     a.seg_n = seg_n.p;
+    a.pair_near = a.n_run > kPairWhole || sel_cap > 0;
     a.dacc = dacc.p;
     a.hbq = hbq.p;
     a.e_fix = e_fix.p;
@@ -345,6 +349,13 @@ template <typename R> class Engine : public EngineBase {
     return a;
   }
 
+  // Up to this many residues the detection pass walks the whole residue pair
+  // list, beside the density pass; above, the near list that pass writes.  A
+  // third of the listed pairs are out of reach, but on 2,000 residues the
+  // detection and hydrogen-bond passes are on the critical path (39 -> 36 us
+  // a step), on 40,000 218 against 223; on 283,000 1,182 against 1,041.
+  static constexpr int kPairWhole = 65536;
+
   // selection records of one evaluation (awsem_debug_selections)
   DBuf<unsigned long long> sel_keys, sel_count;
   long long sel_cap = 0;
@@ -384,10 +395,12 @@ template <typename R> class Engine : public EngineBase {
     CK(cudaStreamCreateWithPriority(&s0, cudaStreamNonBlocking, prio_hi));
     CK(cudaStreamCreateWithPriority(&s1, cudaStreamNonBlocking, prio_lo));
     CK(cudaStreamCreateWithPriority(&s2, cudaStreamNonBlocking, prio_hi));
+    CK(cudaStreamCreateWithPriority(&s3, cudaStreamNonBlocking, prio_hi));
     CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_dens, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_join2, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&ev_join3, cudaEventDisableTiming));
     const Topology &t = in.top;
     int nn = n(), na = natoms();
     res_sys.upload(in.res_sys, s0);
@@ -693,10 +706,6 @@ template <typename R> class Engine : public EngineBase {
     // the emulated lists' decision for this step, before anything reads it
     if (lists_emulated())
       dev::k_list_decide<<<(n_sys() + 127) / 128, 128, 0, s0>>>(nl.p, n_sys(), lst_ago.p, lst_over.p, lst_build.p);
-    // the backbone terms (chain, chi, rama; one kernel of the residue pass)
-    // need only the positions; the recording pass of awsem_debug_selections
-    // runs the whole residue pass instead
-    const bool bb = !a.sel;
     if (fm || fmt || go || px || rx) {
       // fragment memory and the optional terms are independent of the pair
       // passes: second stream
@@ -717,27 +726,50 @@ template <typename R> class Engine : public EngineBase {
       dev::k_pair_sel<R><<<pair_blocks, tb, 0, s0>>>(a, p);
       dev::k_hbond_sel<R><<<hb_blocks, 128, 0, s0>>>(a, p);
     } else {
-      // the backbone terms need only the positions, detection, excluded
-      // volume and the hydrogen-bond terms the positions and the near list:
-      // a third stream, beside fragment memory (second) and the
-      // density-dependent passes (first)
+      // The backbone terms need only the positions: a fourth stream.
+      // Detection, excluded volume and the hydrogen-bond terms need the
+      // positions and a pair list: a third stream, beside fragment memory
+      // (second) and the density-dependent passes (first).
       CK(cudaEventRecord(ev_fork, s0));
-      CK(cudaStreamWaitEvent(s2, ev_fork, 0));
-      if (bb) dev::k_backbone<R><<<nb, tb, 0, s2>>>(a, p);
+      CK(cudaStreamWaitEvent(s3, ev_fork, 0));
+      launch_backbone(a, s3);
+      CK(cudaEventRecord(ev_join3, s3));
+      if (!a.pair_near) CK(cudaStreamWaitEvent(s2, ev_fork, 0));
       dev::k_density<R><<<pair_blocks, tb, 0, s0>>>(a, p);
-      CK(cudaEventRecord(ev_dens, s0));
-      CK(cudaStreamWaitEvent(s2, ev_dens, 0));
+      if (a.pair_near) {
+        CK(cudaEventRecord(ev_dens, s0));
+        CK(cudaStreamWaitEvent(s2, ev_dens, 0));
+      }
       dev::k_pair<R><<<pair_blocks, tb, 0, s2>>>(a, p);
       dev::k_hbond<R><<<hb_blocks, 128, 0, s2>>>(a, p);
       CK(cudaEventRecord(ev_join2, s2));
-      dev::k_residue<R><<<nb, tb, 0, s0>>>(a, p);
+      launch_residue(a, s0);
       dev::k_water_xi<R><<<pair_blocks, tb, 0, s0>>>(a, p);
       dev::k_radial<R><<<pair_blocks, tb, 0, s0>>>(a, p);
       CK(cudaStreamWaitEvent(s0, ev_join2, 0));
+      CK(cudaStreamWaitEvent(s0, ev_join3, 0));
     }
     if (fm || fmt || go || px || rx) CK(cudaStreamWaitEvent(s0, ev_join, 0));
   }
 
+  // The residue and backbone kernels: by tasks while a wave of blocks (four per multiprocessor) covers the residues.
+  // At 17,000 residues (540 blocks) the two take 35 us by tasks and 41 by residues, at 40,000 61 and 44.
+  bool by_tasks() const { return task_blocks() <= 4 * sms_; }
+  void launch_residue(const dev::StepArgs<R> &a, cudaStream_t s)
+  {
+    if (by_tasks())
+      dev::k_residue_tasks<R><<<task_blocks(), 128, 0, s>>>(a, in.ff.p);
+    else
+      dev::k_residue<R><<<(n_run() + dev::kResBlock - 1) / dev::kResBlock, dev::kResBlock, 0, s>>>(a, in.ff.p);
+  }
+  void launch_backbone(const dev::StepArgs<R> &a, cudaStream_t s)
+  {
+    if (by_tasks())
+      dev::k_backbone_tasks<R><<<task_blocks(), 128, 0, s>>>(a, in.ff.p);
+    else
+      dev::k_backbone<R><<<(n_run() + dev::kResBlock - 1) / dev::kResBlock, dev::kResBlock, 0, s>>>(a, in.ff.p);
+  }
+  int task_blocks() const { return (n_run() + dev::kTaskRes - 1) / dev::kTaskRes; }
   int finish_blocks() const { return (n_run() + dev::kFinishRes - 1) / dev::kFinishRes; }
 
   int fm_table_blocks() const
@@ -1302,8 +1334,8 @@ template <typename R> class Engine : public EngineBase {
           case K_NL_DECIDE: dev::k_nl_decide<<<1, 1, 0, s0>>>(nl.p, 0, dstep.p); break;
           case K_NL_BUILD: launch_list_build(a, s0); break;
           case K_DENSITY: dev::k_density<R><<<pair_blocks, tb, 0, s0>>>(a, p); break;
-          case K_RESIDUE: dev::k_residue<R><<<nb, tb, 0, s0>>>(a, p); break;
-          case K_BACKBONE: dev::k_backbone<R><<<nb, tb, 0, s0>>>(a, p); break;
+          case K_RESIDUE: launch_residue(a, s0); break;
+          case K_BACKBONE: launch_backbone(a, s0); break;
           case K_WATER_XI: dev::k_water_xi<R><<<pair_blocks, tb, 0, s0>>>(a, p); break;
           case K_RADIAL: dev::k_radial<R><<<pair_blocks, tb, 0, s0>>>(a, p); break;
           case K_PAIR: dev::k_pair<R><<<pair_blocks, tb, 0, s0>>>(a, p); break;

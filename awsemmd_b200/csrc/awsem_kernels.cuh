@@ -1,6 +1,6 @@
 // Per-step kernels of the AWSEM engine (sm_100a).
 //
-// One MD step is this set of launches (captured into a CUDA graph), on three
+// One MD step is this set of launches (captured into a CUDA graph), on four
 // streams joined before `finish`:
 //   prepare      thread/residue: CA, CB, O -> working copy + virtual N, H, C'
 //                (fix_backbone.cpp:7067-7138) and the contact-bead copy;
@@ -11,14 +11,17 @@
 // first stream:
 //   density      warp/list segment: rho_water, rho_helix (DL1, :7728-7791);
 //                writes the near list
-//   residue      thread/residue: switching functions, burial (SL,
-//                :7795-7841), helical (i,i+4) pairs (:7843-7868), harmonic
-//                bonds, excluded volume inside the residue
+//   residue      thread/residue, or warp/task of 32 residues: switching
+//                functions, burial (SL, :7795-7841), helical (i,i+4) pairs
+//                (:7843-7868)
 //   water_xi     thread/near pair: xi_water (DL2, :7877-7954)
 //   radial       thread/near pair: water/burial/helix radial forces (DL3,
 //                :7956-8057)
+// fourth stream:
+//   backbone     thread/residue, or warp/task of 32 residues: chain, chi,
+//                rama (:2062-2546); harmonic bonds and excluded volume inside
+//                the residue (in the thread/residue form: by residue)
 // third stream:
-//   backbone     thread/residue: chain, chi, rama (:2062-2546)
 //   pair         thread/near pair: DSSP and P_AP detection into queues,
 //                excluded volume between residues (DL3, :8064-8103)
 //   hbond        thread/queued pair: DSSP hydrogen bonds, P_AP
@@ -133,6 +136,7 @@ template <typename R> struct StepArgs {
   // water-xi, pair and hydrogen-bond passes (capacity pcap)
   int2 *pairs, *cpairs;
   int *seg_n;
+  int pair_near;  // the detection pass and its queues: the near list (1), or the whole list (0: no wait for the density pass)
   int *ncount, pcap;
   double4 *cb_build;
   NLState *nl;
@@ -797,102 +801,99 @@ __device__ __forceinline__ void bonds_of(const StepArgs<R> &a, const DevSys<Q> &
   a.e_res[(size_t) E_BOND * s.n_res + r] = e;
 }
 
-// Parts of the per-residue pass: the density-dependent terms (switching,
-// burial, helical pair), the excluded volume inside the residue and the
-// bonds (RES_SL), and the backbone terms chain, chi and rama (RES_BB), which
-// need only the positions and run as their own kernel beside the pair
-// passes.
-constexpr int RES_SL = 1, RES_BB = 2, RES_ALL = 3;
+// The per-residue terms, as tasks that the kernels give to different warps
+// and the persistent step and the recording pass run one after another in one
+// thread.  One thread a residue for all of them was 2,600 (residue) and 3,170
+// (backbone) instructions in series, 14.5 and 15.6 us on 2,000 residues with
+// 132 of the 148 multiprocessors idle.
 
-// SL and the per-residue backbone terms
-template <typename R, bool SEL = false, int PART = RES_ALL>
-__device__ __forceinline__ void residue_one(const StepArgs<R> &a, const FFParams &p, int i, ForceWindow win = {})
+// The residue's burial gammas (fix_backbone.cpp:2887-2899: a phosphorylated
+// residue takes glutamate's)
+template <typename R> __device__ __forceinline__ const double *burial_gammas(const StepArgs<R> &a, int i)
 {
-  DevSys<R> s = a.s;
-  s.win = win;
-  // the per-residue backbone terms (chain, chi, rama, helical pair) are a
-  // small share of the work and some are sums of steep Gaussians: FP64 in
-  // both forms
-  const DevSys<double> sd = widen(s);
-  int n = s.n_res, fl = s.res_flags[i];
-  double *E = a.e_res;
+  return a.s.tables + TB_BURIAL + 3 * ((a.s.res_flags[i] & R_PHOSPH) ? 6 : a.s.res_type[i]);
+}
+
+// one burial well at density rho: its tanh pair
+__device__ __forceinline__ void burial_well(const FFParams &p, double rho, int k, double t[2])
+{
+  t[0] = tanh(p.burial_kappa * (rho - p.burial_ro_min[k]));
+  t[1] = tanh(p.burial_kappa * (p.burial_ro_max[k] - rho));
+}
+
+// SL: water switching function and burial (fix_backbone.cpp:7795-7841), from
+// the three wells' tanh pairs
+template <typename R>
+__device__ __forceinline__ void residue_water(const StepArgs<R> &a, const FFParams &p, int i, const double t[3][2])
+{
+  const DevSys<R> &s = a.s;
   const bool fix = a.groups & G_FIX;
-  if constexpr (PART & RES_SL) {
-  bool water = fix && (p.terms & T_WATER), helix = fix && (p.terms & T_HELIX);
-  double sw = 0, swp = 0, sh = 0, shp = 0;
-  const double rw = density(a, 0, i), rh = density(a, 1, i);
-  a.rho_w[i] = rw;
-  a.rho_h[i] = rh;
-  if (water) switching(rw, p.water_kappa_sigma, p.treshold, sw, swp);
-  if (helix) switching(rh, p.helix_kappa_sigma, p.helix_treshold, sh, shp);
-  a.sig_w[i] = sw;
-  a.sigp_w[i] = swp;
-  a.sig_h[i] = sh;
-  a.sigp_h[i] = shp;
-  double eb = 0.0, bc = 0.0;
+  const double rw = density(a, 0, i);
+  double sw = 0, swp = 0, eb = 0.0, bc = 0.0;
+  if (fix && (p.terms & T_WATER)) switching(rw, p.water_kappa_sigma, p.treshold, sw, swp);
   if (fix && (p.terms & T_BURIAL)) {
-    double rho = rw;
-    // a phosphorylated residue takes glutamate's burial gammas (fix_backbone.cpp:2887-2899)
-    const double *g = s.tables + TB_BURIAL + 3 * ((fl & R_PHOSPH) ? 6 : s.res_type[i]);
-    double t[3][2];
-    for (int k = 0; k < 3; k++) {
-      t[k][0] = tanh(p.burial_kappa * (rho - p.burial_ro_min[k]));
-      t[k][1] = tanh(p.burial_kappa * (p.burial_ro_max[k] - rho));
-      eb += -0.5 * p.k_burial * g[k] * (t[k][0] + t[k][1]);
-    }
+    const double *g = burial_gammas(a, i);
+    for (int k = 0; k < 3; k++) eb += -0.5 * p.k_burial * g[k] * (t[k][0] + t[k][1]);
     bc = g[0] * (t[0][1] * t[0][1] - t[0][0] * t[0][0]);
     bc += g[1] * (t[1][1] * t[1][1] - t[1][0] * t[1][0]);
     bc += g[2] * (t[2][1] * t[2][1] - t[2][0] * t[2][0]);
     bc *= 0.5 * p.k_burial * p.burial_kappa;
   }
+  a.rho_w[i] = rw;
+  a.sig_w[i] = sw;
+  a.sigp_w[i] = swp;
   a.bur[i] = bc;
-  E[(size_t) E_BURIAL * n + i] = eb;
-  // helical (i, i+d) pair; sigma of the partner is recomputed from its density
-  double x1 = 0.0, x2 = 0.0, eh = 0.0;
-  int j = i + p.helix_i_diff;
+  a.e_res[(size_t) E_BURIAL * s.n_res + i] = eb;
+  RadRec &rr = a.rrec[i];
+  rr.sw = sw;
+  rr.bur = bc;
+  rr.sigp = swp;
+  rr.type = s.res_type[i];
+  rr.flags = s.res_flags[i];
+  rr.chain = s.res_chain[i];
+}
+
+// Helix switching function and the helical (i, i + d) pair (:3706-3785,
+// :7843-7868); the partner's sigma is recomputed from its density
+template <typename R, bool SEL = false>
+__device__ __forceinline__ void residue_helix(const StepArgs<R> &a, const DevSys<R> &s, const FFParams &p, int i)
+{
+  const int n = s.n_res;
+  const bool helix = (a.groups & G_FIX) && (p.terms & T_HELIX);
+  const double rh = density(a, 1, i);
+  double sh = 0, shp = 0, x1 = 0.0, x2 = 0.0, eh = 0.0;
+  if (helix) switching(rh, p.helix_kappa_sigma, p.helix_treshold, sh, shp);
+  const int j = i + p.helix_i_diff;
   if (helix && j < n && s.res_chain[j] == s.res_chain[i]) {
     V3<R> d = diff<R>(bead(s, i, B_O), bead(s, j, B_N));
     if (norm2(d) < R(p.helix_cutoff_sq)) {
       double shj, shpj;
       switching(density(a, 1, j), p.helix_kappa_sigma, p.helix_treshold, shj, shpj);
       unsigned gate = 0;
-      eh = (double) helix_pair(sd, p, i, j, sh, shp, shj, shpj, x1, x2, SEL ? &gate : nullptr);
+      eh = (double) helix_pair(widen(s), p, i, j, sh, shp, shj, shpj, x1, x2, SEL ? &gate : nullptr);
       sel_rec<SEL>(a, AWSEM_SEL_HELIX_PAIR, (int) gate, i, j);
     }
   }
+  a.rho_h[i] = rh;
+  a.sig_h[i] = sh;
+  a.sigp_h[i] = shp;
   a.xi1[i] = x1;
   a.xi2[i] = x2;
-  {
-    RadRec &rr = a.rrec[i];
-    rr.sw = sw;
-    rr.bur = bc;
-    rr.x1 = x1;
-    rr.sigp = swp;
-    rr.type = s.res_type[i];
-    rr.flags = fl;
-    rr.chain = s.res_chain[i];
-    // xi2 is read at residue r + helix_i_diff: stored with that residue's
-    // record; a record whose residue r - helix_i_diff is not integrated (no
-    // residue, or a free residue of a serving handle) holds 0
-    if (i + p.helix_i_diff < n) a.rrec[i + p.helix_i_diff].x2 = x2;
-    if (i < p.helix_i_diff || a.res_sys[i - p.helix_i_diff] < 0) rr.x2 = 0.0;
-  }
-  E[(size_t) E_HELIX * n + i] = eh;
-  }
-  if constexpr (PART & RES_BB) {
-  double ec = 0.0, ex = 0.0, er = 0.0;
-  if (fix && (p.terms & T_CHAIN)) ec = (double) chain_term(sd, p, i);
-  bool inner = fix && !(fl & (R_FIRST | R_LAST | R_GLY));
-  if (inner && (p.terms & T_CHI)) ex = (double) chi_term(sd, p, i);
-  if (inner && (p.terms & T_RAMA)) er = (double) rama_term(sd, p, i);
-  E[(size_t) E_CHAIN * n + i] = ec;
-  E[(size_t) E_CHI * n + i] = ex;
-  E[(size_t) E_RAMA * n + i] = er;
-  }
-  if constexpr (PART & RES_SL) {
-  // excluded volume inside the residue (1-3 pairs; 1-2 pairs are excluded)
+  a.rrec[i].x1 = x1;
+  // xi2 is read at residue r + helix_i_diff: stored with that residue's
+  // record; a record whose residue r - helix_i_diff is not integrated (no
+  // residue, or a free residue of a serving handle) holds 0
+  if (j < n) a.rrec[j].x2 = x2;
+  if (i < p.helix_i_diff || a.res_sys[i - p.helix_i_diff] < 0) a.rrec[i].x2 = 0.0;
+  a.e_res[(size_t) E_HELIX * n + i] = eh;
+}
+
+// Excluded volume inside the residue (1-3 pairs; 1-2 pairs are excluded)
+template <typename R, bool SEL = false>
+__device__ __forceinline__ void residue_volume(const StepArgs<R> &a, const DevSys<R> &s, int i)
+{
   double ev = 0.0;
-  unsigned ex_self = (a.groups & G_PAIR) ? a.excl_self[i] : 0x1ffu;
+  const unsigned ex_self = (a.groups & G_PAIR) ? a.excl_self[i] : 0x1ffu;
   for (int b0 = 0; b0 < 3; b0++)
     for (int b1 = b0 + 1; b1 < 3; b1++) {
       if (ex_self & (1u << (b0 * 3 + b1))) continue;
@@ -907,53 +908,219 @@ __device__ __forceinline__ void residue_one(const StepArgs<R> &a, const FFParams
         scatter(s, i, b1, -f.x, -f.y, -f.z);
       }
     }
-  E[(size_t) E_PAIR * n + i] = ev;
-  if (a.groups & G_BOND) bonds_of(a, sd, i);
-  }
+  a.e_res[(size_t) E_PAIR * s.n_res + i] = ev;
+}
+
+// whether the chi and Ramachandran terms apply to residue i
+template <typename R> __device__ __forceinline__ bool residue_inner(const StepArgs<R> &a, int i)
+{
+  return (a.groups & G_FIX) && !(a.s.res_flags[i] & (R_FIRST | R_LAST | R_GLY));
+}
+// The chain and chi terms run in FP64 in both forms, as the Ramachandran and
+// helical ones: a small share of the work, and some are sums of steep Gaussians.
+template <typename R>
+__device__ __forceinline__ void residue_chain(const StepArgs<R> &a, const DevSys<double> &s, const FFParams &p, int i)
+{
+  double e = 0.0;
+  if ((a.groups & G_FIX) && (p.terms & T_CHAIN)) e = chain_term(s, p, i);
+  a.e_res[(size_t) E_CHAIN * s.n_res + i] = e;
+}
+template <typename R>
+__device__ __forceinline__ void residue_chi(const StepArgs<R> &a, const DevSys<double> &s, const FFParams &p, int i)
+{
+  double e = 0.0;
+  if (residue_inner(a, i) && (p.terms & T_CHI)) e = chi_term(s, p, i);
+  a.e_res[(size_t) E_CHI * s.n_res + i] = e;
+}
+
+// The tasks of one residue by one thread, forces to the window of s when it
+// has one: the density-dependent ones with the bonds and the excluded volume
+// inside the residue, and the backbone ones.
+template <typename R, bool SEL = false>
+__device__ __forceinline__ void residue_density(const StepArgs<R> &a, const DevSys<R> &s, const FFParams &p, int i)
+{
+  double t[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+  if ((a.groups & G_FIX) && (p.terms & T_BURIAL))
+    for (int k = 0; k < 3; k++) burial_well(p, density(a, 0, i), k, t[k]);
+  residue_water(a, p, i, t);
+  residue_helix<R, SEL>(a, s, p, i);
+  residue_volume<R, SEL>(a, s, i);
+  if (a.groups & G_BOND) bonds_of(a, widen(s), i);
+}
+template <typename R>
+__device__ __forceinline__ void residue_backbone(const StepArgs<R> &a, const DevSys<R> &s, const FFParams &p, int i)
+{
+  const DevSys<double> sd = widen(s);
+  residue_chain(a, sd, p, i);
+  residue_chi(a, sd, p, i);
+  double er = 0.0;
+  if (residue_inner(a, i) && (p.terms & T_RAMA)) er = rama_term(sd, p, i);
+  a.e_res[(size_t) E_RAMA * s.n_res + i] = er;
 }
 
 template <typename R, bool SEL = false> __device__ __forceinline__ void residue_pass(const StepArgs<R> &a, const FFParams &p, Span sp)
 {
   for (int i = sp.t; i < a.n_run; i += sp.nthr)
-    if (a.res_sys[i] >= 0) residue_one<R, SEL>(a, p, i);
+    if (a.res_sys[i] >= 0) {
+      residue_density<R, SEL>(a, a.s, p, i);
+      residue_backbone(a, a.s, p, i);
+    }
+}
+template <typename R> __global__ void __launch_bounds__(128) k_residue_sel(StepArgs<R> a, FFParams p)
+{
+  residue_pass<R, true>(a, p, grid_span());
 }
 
-// The standalone residue kernel: 128 residues per block and iteration; the
-// forces its terms push to residues r0 - 1 .. r0 + 127 + helix_i_diff (the
-// helical pair reaches i + 4) are summed in shared memory and flushed with
-// one global atomic per non-zero component.  Each contribution is converted
-// to fixed point before it is summed, so the result is the direct scatter's
-// bit for bit.
-constexpr int kResBlock = 128, kResHalo = 5, kResWin = kResBlock + kResHalo;
-template <typename R, bool SEL, int PART> __device__ __forceinline__ void residue_pass_window(const StepArgs<R> &a, const FFParams &p)
+// A block's shared force window over residues [r0, r0 + n): each contribution
+// is converted to fixed point before it is summed there, and the flush adds
+// one global atomic per non-zero component, so the result is the direct
+// scatter's bit for bit.
+__device__ __forceinline__ void window_clear(unsigned long long *acc, int n)
 {
-  __shared__ unsigned long long acc[kResWin * 9];
+  for (int k = threadIdx.x; k < 9 * n; k += blockDim.x) acc[k] = 0ull;
+}
+__device__ __forceinline__ void window_flush(const unsigned long long *acc, int n, int r0, int n_res,
+                                             unsigned long long *facc)
+{
+  for (int k = threadIdx.x; k < 9 * n; k += blockDim.x) {
+    const unsigned long long v = acc[k];
+    const int r = r0 + k / 9;
+    if (v && r >= 0 && r < n_res) atomicAdd(facc + (size_t) 9 * r + k % 9, v);
+  }
+}
+
+// Two forms of the residue and backbone kernels.  A thread per residue fills
+// the chip at full load (283,000 residues: 71 and 78 us).  A warp per task of
+// 32 residues shortens the series where a wave of blocks covers the residues:
+// on 2,000 the step went from 51 to 36 us.  At full load its warps wait for
+// their block's longest task (backbone 238 us), so the engine picks by size.
+constexpr int kResBlock = 128, kResHalo = 5;  // the helical pair reaches i + 4
+template <typename R> __global__ void __launch_bounds__(kResBlock, 4) k_residue(StepArgs<R> a, FFParams p)
+{
+  constexpr int kWin = kResBlock + kResHalo;
+  __shared__ unsigned long long acc[kWin * 9];
   const uint32_t addr = (uint32_t) __cvta_generic_to_shared(acc);
   for (int r0 = blockIdx.x * kResBlock; r0 < a.n_run; r0 += gridDim.x * kResBlock) {
-    for (int k = threadIdx.x; k < kResWin * 9; k += kResBlock) acc[k] = 0ull;
+    window_clear(acc, kWin);
     __syncthreads();
     const int i = r0 + threadIdx.x;
-    if (i < a.n_run && a.res_sys[i] >= 0) residue_one<R, SEL, PART>(a, p, i, ForceWindow{addr, r0 - 1, kResWin});
+    DevSys<R> s = a.s;
+    s.win = ForceWindow{addr, r0 - 1, kWin};
+    if (i < a.n_run && a.res_sys[i] >= 0) residue_density(a, s, p, i);
     __syncthreads();
-    for (int k = threadIdx.x; k < kResWin * 9; k += kResBlock) {
-      const unsigned long long v = acc[k];
-      const int r = r0 - 1 + k / 9;
-      if (v && r >= 0 && r < a.s.n_res) atomicAdd(a.s.facc + (size_t) 9 * r + k % 9, v);
+    window_flush(acc, kWin, r0 - 1, a.s.n_res, a.s.facc);
+    __syncthreads();
+  }
+}
+template <typename R> __global__ void __launch_bounds__(kResBlock, 4) k_backbone(StepArgs<R> a, FFParams p)
+{
+  constexpr int kWin = kResBlock + 2;
+  __shared__ unsigned long long acc[kWin * 9];
+  const uint32_t addr = (uint32_t) __cvta_generic_to_shared(acc);
+  for (int r0 = blockIdx.x * kResBlock; r0 < a.n_run; r0 += gridDim.x * kResBlock) {
+    window_clear(acc, kWin);
+    __syncthreads();
+    const int i = r0 + threadIdx.x;
+    DevSys<R> s = a.s;
+    s.win = ForceWindow{addr, r0 - 1, kWin};
+    if (i < a.n_run && a.res_sys[i] >= 0) residue_backbone(a, s, p, i);
+    __syncthreads();
+    window_flush(acc, kWin, r0 - 1, a.s.n_res, a.s.facc);
+    __syncthreads();
+  }
+}
+
+// The density-dependent tasks, 32 residues a block: a warp each for the water
+// switching function with the first burial well, the other two wells, and the
+// helix function with the helical pair.  Bound by the latency of its FP64
+// hyperbolic tangents: at most three in series a warp instead of ten.
+constexpr int kTaskRes = 32;  // residues per block of the task kernels (128 threads)
+template <typename R> __global__ void __launch_bounds__(128) k_residue_tasks(StepArgs<R> a, FFParams p)
+{
+  __shared__ double well[2][2][kTaskRes];
+  const int task = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool burial = (a.groups & G_FIX) && (p.terms & T_BURIAL);
+  for (int r0 = blockIdx.x * kTaskRes; r0 < a.n_run; r0 += gridDim.x * kTaskRes) {
+    const int i = r0 + lane;
+    const bool on = i < a.n_run && a.res_sys[i] >= 0;
+    double t[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+    if (on) {
+      if (task == 3)
+        residue_helix(a, a.s, p, i);
+      else if (burial)
+        burial_well(p, density(a, 0, i), task, t[0]);
+    }
+    if (task == 1 || task == 2) {
+      well[task - 1][0][lane] = t[0][0];
+      well[task - 1][1][lane] = t[0][1];
+    }
+    __syncthreads();
+    if (task == 0 && on) {
+#pragma unroll
+      for (int k = 1; k < 3; k++) t[k][0] = well[k - 1][0][lane], t[k][1] = well[k - 1][1][lane];
+      residue_water(a, p, i, t);
     }
     __syncthreads();
   }
 }
-template <typename R> __global__ void __launch_bounds__(kResBlock, 4) k_residue(StepArgs<R> a, FFParams p)
+
+// The tasks that need only the positions, 32 residues a block: a warp each
+// for chain with the excluded volume inside the residue, chi with the bonds,
+// and the phi and psi halves of the Ramachandran term, which meet in shared
+// memory.
+constexpr int kTaskWin = kTaskRes + 2;
+template <typename R> __global__ void __launch_bounds__(128, 4) k_backbone_tasks(StepArgs<R> a, FFParams p)
 {
-  residue_pass_window<R, false, RES_SL>(a, p);
-}
-template <typename R> __global__ void __launch_bounds__(kResBlock, 4) k_backbone(StepArgs<R> a, FFParams p)
-{
-  residue_pass_window<R, false, RES_BB>(a, p);
-}
-template <typename R> __global__ void __launch_bounds__(kResBlock) k_residue_sel(StepArgs<R> a, FFParams p)
-{
-  residue_pass_window<R, true, RES_ALL>(a, p);
+  __shared__ unsigned long long acc[kTaskWin * 9];
+  __shared__ double ang[2][2][kTaskRes], half[16][kTaskRes];
+  const uint32_t addr = (uint32_t) __cvta_generic_to_shared(acc);
+  const int task = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r0 = blockIdx.x * kTaskRes; r0 < a.n_run; r0 += gridDim.x * kTaskRes) {
+    window_clear(acc, kTaskWin);
+    __syncthreads();
+    const int i = r0 + lane;
+    const bool on = i < a.n_run && a.res_sys[i] >= 0;
+    DevSys<R> s = a.s;
+    s.win = ForceWindow{addr, r0 - 1, kTaskWin};
+    const DevSys<double> sd = widen(s);
+    const bool rama = on && residue_inner(a, i) && (p.terms & T_RAMA);
+    V3<double> sl[5];
+    if (task == 0 && on) {
+      residue_chain(a, sd, p, i);
+      residue_volume(a, s, i);
+    } else if (task == 1 && on) {
+      residue_chi(a, sd, p, i);
+      if (a.groups & G_BOND) bonds_of(a, sd, i);
+    } else if (task >= 2 && rama) {
+      dihedral(sd, p, i, task == 2, ang[task - 2][0][lane], ang[task - 2][1][lane], sl);
+    }
+    __syncthreads();
+    double g[2] = {0.0, 0.0}, er = 0.0;
+    if (task >= 2 && rama) {
+      er = rama_wells(sd, p, i, ang[0][0][lane], ang[0][1][lane], ang[1][0][lane], ang[1][1][lane], g[0], g[1]);
+      if (task == 3) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+          half[3 * k][lane] = g[1] * sl[k].x;
+          half[3 * k + 1][lane] = g[1] * sl[k].y;
+          half[3 * k + 2][lane] = g[1] * sl[k].z;
+        }
+      }
+    }
+    __syncthreads();
+    if (task == 2 && on) {
+      if (rama && (g[0] != 0.0 || g[1] != 0.0)) {
+#pragma unroll
+        for (int k = 0; k < 5; k++)
+          scatter(sd, k == 0 || k == 3 ? i - 1 : k == 2 ? i + 1 : i, k < 3 ? B_CA : B_O, g[0] * sl[k].x + half[3 * k][lane],
+                  g[0] * sl[k].y + half[3 * k + 1][lane], g[0] * sl[k].z + half[3 * k + 2][lane]);
+      }
+      a.e_res[(size_t) E_RAMA * s.n_res + i] = er;
+    }
+    __syncthreads();
+    window_flush(acc, kTaskWin, r0 - 1, a.s.n_res, a.s.facc);
+    __syncthreads();
+  }
 }
 
 // DL2: water-mediated density derivative coefficients (fix_backbone.cpp:
@@ -1137,7 +1304,10 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void pair_pas
   const int pap_sep = min(p.i_med_min + 2 * p.i_diff_pap, p.i_med_max + 1);
   const size_t qd = 0, qp = (size_t) 2 * a.pcap;  // queue regions: DSSP (both orientations), P_AP
   unsigned long long *e_ev = (unsigned long long *) a.e_fix + (size_t) 4 * n;
-  const int lane = threadIdx.x & 31, seg = a.nl->seg_len, np = a.nl->nseg * seg;
+  const bool near = a.pair_near;
+  const int2 *const list = near ? a.cpairs : a.pairs;
+  const int npairs = min(a.nl->npairs, a.pcap);
+  const int lane = threadIdx.x & 31, seg = near ? a.nl->seg_len : 1, np = near ? a.nl->nseg * seg : npairs;
   // Queue entries are staged per warp in shared memory and written out 32 at
   // a time with one atomic reservation: one counter update per 32 entries
   // instead of one per warp iteration (same-address atomics serialise in L2).
@@ -1187,7 +1357,7 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void pair_pas
     int i = 0, j = 0, sh = 9;
     float dca = 0.f;
     if (q >= 0) {
-      const int2 ij = a.cpairs[q];
+      const int2 ij = list[q];
       i = ij.x, j = ij.y;
       const bool shortr = s.res_chain[j] == s.res_chain[i] && j - i < 5;
       sh = shortr ? 0 : 9;
@@ -1242,11 +1412,11 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void pair_pas
   // warp-uniform trip count: the queue appends below are warp collectives
   // (a warp's 32 indices lie in one near-list segment: segments are multiples of 32 long)
   for (int base = sp.t - lane; base < np; base += sp.nthr) {
-    const int q = base + lane, sg = base / seg, have = a.seg_n[sg] - (base - sg * seg);
+    const int q = base + lane, sg = base / seg, have = near ? a.seg_n[sg] - (base - sg * seg) : np - base;
     if (have <= 0) continue;  // warp-uniform: past this segment's near pairs
     bool q_d0 = false, q_d1 = false, q_p = false, q_e = false;  // queue: DSSP O(i), DSSP O(j), P_AP; stage: EV
     if (lane < have) {
-    const int2 ij = a.cpairs[q];
+    const int2 ij = list[q];
     const int i = ij.x, j = ij.y;
     // (the topology arrays, not the residue pass's records: this pass runs
     // beside the residue pass)
@@ -1307,10 +1477,11 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void hbond_pa
 {
   const DevSys<R> &s = a.s;
   const int nd = a.nl->n_dssp, np = a.nl->n_pap, n = s.n_res;
+  const int2 *const list = a.pair_near ? a.cpairs : a.pairs;
   for (int t = sp.t; t < nd + np; t += sp.nthr) {
     const bool d = t < nd;
     const int q = d ? a.hbq[t] : a.hbq[(size_t) 2 * a.pcap + (t - nd)];
-    const int2 ij = a.cpairs[q < 0 ? ~q : q];
+    const int2 ij = list[q < 0 ? ~q : q];
     const int i = q < 0 ? ij.y : ij.x, j = q < 0 ? ij.x : ij.y;
     unsigned gate = 0;
     const R e = d ? dssp_term(s, p, i, j, SEL ? &gate : nullptr) : pap_term(s, p, i, j, SEL ? &gate : nullptr);
