@@ -628,7 +628,7 @@ template <typename R> class Engine : public EngineBase {
     CK(cudaMemcpyAsync(nl.p, &st, sizeof st, cudaMemcpyHostToDevice, s0));
   }
 
-  // cell grids of the large replicas (see k_grid_setup)
+  // cell grids of the large replicas (see k_grid_build)
   DBuf<int> big_rep, big_of, cell_count, cell_start, cell_fill, res_cell, sorted_res;
   DBuf<dev::GridDesc> grid_desc;
   int nbig = 0;
@@ -670,24 +670,18 @@ template <typename R> class Engine : public EngineBase {
 
   void launch_list_build(const dev::StepArgs<R> &a, cudaStream_t s)
   {
-    const int nn = n_run(), tb = 128, nb = (nn + tb - 1) / tb;
+    const int nn = n_run(), tb = 128;
     const int wb = std::min((nn * 32 + tb - 1) / tb, 8 * sms_);
     const dev::GridArgs g = grid_args();
-    if (nbig) {
-      dev::k_grid_setup<R><<<nbig, 256, 0, s>>>(a, g);
-      dev::k_grid_count<R><<<nb, tb, 0, s>>>(a, g);
-      dev::k_grid_scan<R><<<nbig, 1024, 0, s>>>(a, g);
-      dev::k_grid_fill<R><<<nb, tb, 0, s>>>(a, g);
-    }
+    if (nbig) dev::k_grid_build<R><<<nbig, dev::kGridThreads, 0, s>>>(a, g);
     dev::k_nl_build<R><<<wb, tb, 0, s>>>(a, g, nn);
   }
 
   void launch_prepare_and_list(const dev::StepArgs<R> &a, cudaStream_t s, bool force, bool advance)
   {
     const FFParams &p = in.ff.p;
-    const int nn = n_run(), tb = 128, nb = (nn + tb - 1) / tb;
-    dev::k_prepare<R><<<nb, tb, 0, s>>>(a, p);
-    dev::k_nl_decide<<<1, 1, 0, s>>>(nl.p, force ? 1 : 0, advance ? dstep.p : nullptr);
+    const int tb = dev::kPrepBlock, nb = (n_run() + tb - 1) / tb;
+    dev::k_prepare<R><<<nb, tb, 0, s>>>(a, p, force ? 1 : 0, advance ? dstep.p : nullptr);
     launch_list_build(a, s);
   }
 
@@ -1330,8 +1324,8 @@ template <typename R> class Engine : public EngineBase {
       for (int k = 0; k < AWSEM_NKERNELS; k++) {
         CK(cudaEventRecord(ev[2 * k], s0));
         switch (k) {
-          case K_PREPARE: dev::k_prepare<R><<<nb, tb, 0, s0>>>(a, p); break;
-          case K_NL_DECIDE: dev::k_nl_decide<<<1, 1, 0, s0>>>(nl.p, 0, dstep.p); break;
+          case K_PREPARE: dev::k_prepare<R><<<nb, tb, 0, s0>>>(a, p, 0, dstep.p); break;
+          case K_NL_DECIDE: break;  // taken by the last block of k_prepare
           case K_NL_BUILD: launch_list_build(a, s0); break;
           case K_DENSITY: dev::k_density<R><<<pair_blocks, tb, 0, s0>>>(a, p); break;
           case K_RESIDUE: launch_residue(a, s0); break;

@@ -4,8 +4,8 @@
 // streams joined before `finish`:
 //   prepare      thread/residue: CA, CB, O -> working copy + virtual N, H, C'
 //                (fix_backbone.cpp:7067-7138) and the contact-bead copy;
-//                zero forces; list-check data
-//   nl_decide    1 thread: rebuild decision for the residue pair list
+//                zero forces; list-check data; the last block decides whether
+//                the residue pair list is rebuilt
 //   nl_build     warp/residue: pairs i < j of contact beads within the list
 //                radius, appended to a flat pair array
 // first stream:
@@ -96,6 +96,7 @@ struct NLState {
   alignas(128) int n_dssp;  // hydrogen-bond queue lengths of the current evaluation
   alignas(128) int n_pap;
   alignas(128) int fm_next;  // fragment-memory work units handed out (k_fragmem), zeroed by the list decision
+  alignas(128) int prepared;  // blocks of k_prepare that are done (zero between launches)
   alignas(128) int end_pad;
 };
 
@@ -223,135 +224,161 @@ __device__ __forceinline__ void atomic_max_f(float *addr, float v)
   atomicMax((int *) addr, __float_as_int(v));
 }
 
-template <typename R> __device__ __forceinline__ void prepare_pass(const StepArgs<R> &a, const FFParams &p, Span sp)
+// maximum over the warp of non-negative floats (they order like their bits)
+__device__ __forceinline__ float warp_max(float v)
 {
-  float d2 = 0.f, dl = 0.f;
-  // squared bead offsets, maximised over this thread's residues; the square
-  // root of the maximum is the maximum of the square roots (both roundings
-  // are monotonic), so one root per thread gives the same maxima
-  double qO = 0.0, qN = 0.0, qCA = 0.0, qAll = 0.0, qB = 0.0, qX = 0.0, qNCA = 0.0;
-  const int lane = threadIdx.x & 31;
-  // warp-uniform trip count: the maxima are reduced across the warp below
-  for (int r0 = sp.t - lane; r0 < a.n_run; r0 += sp.nthr) {
-  const int r = r0 + lane;
-  if (r < a.n_run) {
-    unsigned long long *f = a.s.facc + (size_t) 9 * r;
-    for (int k = 0; k < 9; k++) f[k] = 0ull;
-    for (int k = 0; k < a.efix_slots; k++) a.e_fix[(size_t) k * a.s.n_res + r] = 0;
-    for (int k = 0; k < 3; k++) a.dacc[(size_t) k * a.s.n_res + r] = 0;
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+
+// The prepare pass of BLOCK residues by a block of BLOCK threads, in parts: a
+// residue's working coordinates from its and its neighbours' positions (which
+// come through shared memory), the list-check maxima, and the stores.  The
+// bead offsets stay squared in FP32, rounded up, until one root per block and
+// quantity: they only bound the list's validity.
+template <typename R, int BLOCK> struct PrepareTile {
+  // maxima over this thread's residues: squared displacement and bead offsets
+  enum { M_D2, M_O, M_N, M_CA, M_ALL, M_OX, M_NCA, M_LIST, M_CBX, M_COUNT };
+  float q[M_COUNT];
+  double ca[3], cb[3], o[3], n[3], h[3], cp[3];
+  bool on, gly, over;
+
+  __device__ __forceinline__ PrepareTile()
+  {
+#pragma unroll
+    for (int k = 0; k < M_COUNT; k++) q[k] = 0.f;
   }
-  if (r < a.n_run && a.res_sys[r] >= 0) {
-    const double *x = a.x;
-    int fl = a.s.res_flags[r];
-    double ca[3], cb[3], o[3], n[3] = {0, 0, 0}, h[3] = {0, 0, 0}, cp[3] = {0, 0, 0};
-    bool finite = true;
-    for (int k = 0; k < 3; k++) {
-      ca[k] = x[(3 * r + 0) * 3 + k];
-      cb[k] = x[(3 * r + 1) * 3 + k];
-      o[k] = x[(3 * r + 2) * 3 + k];
-      finite = finite && isfinite(ca[k]) && isfinite(cb[k]) && isfinite(o[k]);
+  __device__ __forceinline__ void up(int k, double v) { q[k] = fmaxf(q[k], __double2float_ru(v)); }
+
+  __device__ __forceinline__ void compute(const StepArgs<R> &a, const FFParams &p, int r0, double *sx)
+  {
+    const int r = r0 + (int) threadIdx.x, here = min(BLOCK, a.n_run - r0);
+    on = r < a.n_run && a.res_sys[r] >= 0;
+    const int fl = on ? a.s.res_flags[r] : 0;
+    const double4 b0 = on ? a.cb_build[r] : make_double4(0, 0, 0, 0);
+    for (int k = threadIdx.x; k < (here + 2) * 9; k += BLOCK) {
+      const long long e = 9ll * (r0 - 1) + k;
+      sx[k] = e >= 0 && e < 9ll * a.s.n_res ? a.x[e] : 0.0;
     }
-    if (!finite) a.nl->bad_x = 1;
-    if (!(fl & R_FIRST)) {
-      for (int k = 0; k < 3; k++) {
-        double ca0 = x[(3 * (r - 1) + 0) * 3 + k], o0 = x[(3 * (r - 1) + 2) * 3 + k];
+    __syncthreads();
+    gly = fl & R_GLY;
+    over = false;
+    const double *x = sx + 9 * (threadIdx.x + 1);  // this residue; the one before at x - 9, after at x + 9
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      ca[k] = x[k];
+      cb[k] = x[3 + k];
+      o[k] = x[6 + k];
+      n[k] = h[k] = cp[k] = 0.0;
+      if (!(fl & R_FIRST)) {
+        const double ca0 = x[k - 9], o0 = x[6 + k - 9];
         n[k] = __dadd_rn(__dadd_rn(__dmul_rn(p.an, ca0), __dmul_rn(p.bn, ca[k])), __dmul_rn(p.cn, o0));
         h[k] = __dadd_rn(__dadd_rn(__dmul_rn(p.ah, ca0), __dmul_rn(p.bh, ca[k])), __dmul_rn(p.ch, o0));
       }
+      if (!(fl & R_LAST))
+        cp[k] = __dadd_rn(__dadd_rn(__dmul_rn(p.ap, ca[k]), __dmul_rn(p.bp, x[k + 9])), __dmul_rn(p.cp, o[k]));
     }
-    if (!(fl & R_LAST)) {
-      for (int k = 0; k < 3; k++) {
-        double ca1 = x[(3 * (r + 1) + 0) * 3 + k];
-        cp[k] = __dadd_rn(__dadd_rn(__dmul_rn(p.ap, ca[k]), __dmul_rn(p.bp, ca1)), __dmul_rn(p.cp, o[k]));
+    if (on) {
+      bool finite = true;
+#pragma unroll
+      for (int k = 0; k < 3; k++) finite = finite && isfinite(ca[k]) && isfinite(cb[k]) && isfinite(o[k]);
+      if (!finite) a.nl->bad_x = 1;
+      if (a.lst_x0) {
+        // LAMMPS check_distance for the emulated lists: an atom farther than
+        // half the skin from where it was at the last build
+        const double trig = 0.25 * a.nl->lst_skin * a.nl->lst_skin;
+        const double *h0 = a.lst_x0 + (size_t) 9 * r;
+        for (int b = 0; b < 3; b++) {
+          const double dx = x[3 * b] - h0[3 * b], dy = x[3 * b + 1] - h0[3 * b + 1], dz = x[3 * b + 2] - h0[3 * b + 2];
+          const double d2b = dx * dx + dy * dy + dz * dz;
+          if (d2b > trig) over = true;
+          if (b == 0) q[M_LIST] = fmaxf(q[M_LIST], (float) d2b * 1.0001f);
+        }
+      }
+      auto dist2 = [](const double *u, const double *v) {
+        const double ex = u[0] - v[0], ey = u[1] - v[1], ez = u[2] - v[2];
+        return ex * ex + ey * ey + ez * ez;
+      };
+      // list-validity data: contact-bead displacement and bead offsets, and
+      // the reach of the residue's beads around its CA (excluded volume)
+      double c[3];
+#pragma unroll
+      for (int k = 0; k < 3; k++) c[k] = gly ? ca[k] : cb[k];
+      const double b0v[3] = {b0.x, b0.y, b0.z};
+      const double o_o = dist2(o, c), o_ca = dist2(ca, c);
+      up(M_D2, dist2(c, b0v));
+      up(M_O, o_o);
+      up(M_CA, o_ca);
+      up(M_ALL, fmax(fmax(o_ca, dist2(cb, c)), o_o));
+      up(M_CBX, dist2(cb, ca));
+      up(M_OX, dist2(o, ca));
+      if (!(fl & R_FIRST)) {
+        up(M_N, dist2(n, c));
+        up(M_NCA, dist2(n, ca));
       }
     }
-    if (a.lst_x0) {
-      // LAMMPS check_distance for the emulated lists: an atom farther than
-      // half the skin from where it was at the last build
-      const double trig = 0.25 * a.nl->lst_skin * a.nl->lst_skin;
-      const double *h = a.lst_x0 + (size_t) 9 * r;
-      bool over = false;
-      for (int b = 0; b < 3; b++) {
-        const double *q = b == 0 ? ca : b == 1 ? cb : o;
-        const double dx = q[0] - h[3 * b], dy = q[1] - h[3 * b + 1], dz = q[2] - h[3 * b + 2];
-        const double d2b = dx * dx + dy * dy + dz * dz;
-        if (d2b > trig) over = true;
-        if (b == 0) dl = fmaxf(dl, (float) d2b * 1.0001f);
-      }
+    __syncthreads();  // every thread has read its neighbours
+  }
+
+  // working coordinates, contact bead, cleared accumulators
+  __device__ __forceinline__ void store(const StepArgs<R> &a, int r0) const
+  {
+    const int r = r0 + (int) threadIdx.x, here = min(BLOCK, a.n_run - r0);
+    if (on) {
+      double4 *w = const_cast<double4 *>(a.s.pos) + (size_t) r * N_BEADS;
+      w[B_CA] = make_double4(ca[0], ca[1], ca[2], 0.0);
+      w[B_CB] = make_double4(cb[0], cb[1], cb[2], 0.0);
+      w[B_O] = make_double4(o[0], o[1], o[2], 0.0);
+      w[B_N] = make_double4(n[0], n[1], n[2], 0.0);
+      w[B_H] = make_double4(h[0], h[1], h[2], 0.0);
+      w[B_CP] = make_double4(cp[0], cp[1], cp[2], 0.0);
+      const_cast<double4 *>(a.s.cpos)[r] =
+          gly ? make_double4(ca[0], ca[1], ca[2], 0.0) : make_double4(cb[0], cb[1], cb[2], 0.0);
       if (over) a.lst_over[a.res_sys[r]] = 1;
     }
-    double4 *w = const_cast<double4 *>(a.s.pos) + (size_t) r * N_BEADS;
-    w[B_CA] = make_double4(ca[0], ca[1], ca[2], 0.0);
-    w[B_CB] = make_double4(cb[0], cb[1], cb[2], 0.0);
-    w[B_O] = make_double4(o[0], o[1], o[2], 0.0);
-    w[B_N] = make_double4(n[0], n[1], n[2], 0.0);
-    w[B_H] = make_double4(h[0], h[1], h[2], 0.0);
-    w[B_CP] = make_double4(cp[0], cp[1], cp[2], 0.0);
-    {
-      const double *cc = (fl & R_GLY) ? ca : cb;
-      const_cast<double4 *>(a.s.cpos)[r] = make_double4(cc[0], cc[1], cc[2], 0.0);
-    }
-    {
-      // reach of the residue's beads around its CA (excluded-volume prefilter)
-      double ux = cb[0] - ca[0], uy = cb[1] - ca[1], uz = cb[2] - ca[2];
-      double wx = o[0] - ca[0], wy = o[1] - ca[1], wz = o[2] - ca[2];
-      qB = fmax(qB, ux * ux + uy * uy + uz * uz);
-      qX = fmax(qX, wx * wx + wy * wy + wz * wz);
-    }
-    // list-validity data: contact-bead displacement and bead offsets
-    const double *c = (fl & R_GLY) ? ca : cb;
-    double4 b0 = a.cb_build[r];
-    double dx = c[0] - b0.x, dy = c[1] - b0.y, dz = c[2] - b0.z;
-    d2 = fmaxf(d2, (float) (dx * dx + dy * dy + dz * dz));
-    auto off2 = [&](const double *q) {
-      double ex = q[0] - c[0], ey = q[1] - c[1], ez = q[2] - c[2];
-      return ex * ex + ey * ey + ez * ez;
-    };
-    const double o_o = off2(o), o_ca = off2(ca);
-    qO = fmax(qO, o_o);
-    qCA = fmax(qCA, o_ca);
-    qAll = fmax(qAll, fmax(fmax(o_ca, off2(cb)), o_o));
-    if (!(fl & R_FIRST)) {
-      qN = fmax(qN, off2(n));
-      const double ex = n[0] - ca[0], ey = n[1] - ca[1], ez = n[2] - ca[2];
-      qNCA = fmax(qNCA, ex * ex + ey * ey + ez * ez);
+    for (int k = threadIdx.x; k < 9 * here; k += BLOCK) a.s.facc[(size_t) 9 * r0 + k] = 0ull;
+    if (r < a.n_run) {
+      for (int k = 0; k < a.efix_slots; k++) a.e_fix[(size_t) k * a.s.n_res + r] = 0;
+#pragma unroll
+      for (int k = 0; k < 3; k++) a.dacc[(size_t) k * a.s.n_res + r] = 0;
     }
   }
-  }
-  float oO = (float) sqrt(qO), oN = (float) sqrt(qN), oCA = (float) sqrt(qCA), oAll = (float) sqrt(qAll);
-  float oB = (float) sqrt(qB), oX = (float) sqrt(qX), oNCA = (float) sqrt(qNCA);
-  // warp max, block max, then one atomic per block and quantity (every
-  // thread of the block calls this pass)
-  for (int s = 16; s > 0; s >>= 1) {
-    d2 = fmaxf(d2, __shfl_xor_sync(0xffffffffu, d2, s));
-    oO = fmaxf(oO, __shfl_xor_sync(0xffffffffu, oO, s));
-    oN = fmaxf(oN, __shfl_xor_sync(0xffffffffu, oN, s));
-    oCA = fmaxf(oCA, __shfl_xor_sync(0xffffffffu, oCA, s));
-    oAll = fmaxf(oAll, __shfl_xor_sync(0xffffffffu, oAll, s));
-    oB = fmaxf(oB, __shfl_xor_sync(0xffffffffu, oB, s));
-    oX = fmaxf(oX, __shfl_xor_sync(0xffffffffu, oX, s));
-    oNCA = fmaxf(oNCA, __shfl_xor_sync(0xffffffffu, oNCA, s));
-    dl = fmaxf(dl, __shfl_xor_sync(0xffffffffu, dl, s));
-  }
-  __shared__ float red[9][32];
-  if (lane == 0) {
-    const int w = threadIdx.x >> 5;
-    red[0][w] = d2, red[1][w] = oO, red[2][w] = oN, red[3][w] = oCA, red[4][w] = oAll, red[5][w] = oX;
-    red[6][w] = oNCA, red[7][w] = dl, red[8][w] = oB;
-  }
-  __syncthreads();
-  if (threadIdx.x < 9) {
-    const int k = threadIdx.x;
-    float m = 0.f;
-    for (int w = 0; w < (int) (blockDim.x >> 5); w++) m = fmaxf(m, red[k][w]);
-    float *dst = k == 0 ? &a.nl->d2max : k == 1 ? &a.nl->bO : k == 2 ? &a.nl->bN : k == 3 ? &a.nl->bCA
-               : k == 4 ? &a.nl->bAll : k == 5 ? &a.nl->bOx : k == 6 ? &a.nl->bNCA : k == 7 ? &a.nl->lst_d2max
-               : &a.nl->bCBx;
-    if (m > 0.f) atomic_max_f(dst, m);  // the maxima start each step at 0
-  }
-}
 
-template <typename R> __global__ void k_prepare(StepArgs<R> a, FFParams p) { prepare_pass(a, p, grid_span()); }
+  // warp max, block max, then one atomic per block and quantity, by threads of the first warp
+  __device__ __forceinline__ void reduce(NLState *nl)
+  {
+    __shared__ float red[M_COUNT][BLOCK / 32];
+#pragma unroll
+    for (int k = 0; k < M_COUNT; k++) {
+      const float m = warp_max(q[k]);
+      if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x < M_COUNT) {
+      const int k = threadIdx.x;
+      float m = red[k][0];
+#pragma unroll
+      for (int w = 1; w < BLOCK / 32; w++) m = fmaxf(m, red[k][w]);
+      if (k != M_D2 && k != M_LIST) m = __fsqrt_ru(m);
+      float *dst = k == M_D2 ? &nl->d2max : k == M_O ? &nl->bO : k == M_N ? &nl->bN : k == M_CA ? &nl->bCA
+                 : k == M_ALL ? &nl->bAll : k == M_OX ? &nl->bOx : k == M_NCA ? &nl->bNCA : k == M_LIST ? &nl->lst_d2max
+                 : &nl->bCBx;
+      if (m > 0.f) atomic_max_f(dst, m);  // the maxima start each step at 0
+    }
+  }
+};
+
+// the whole pass by a grid of any size (the persistent step)
+template <typename R, int BLOCK>
+__device__ __forceinline__ void prepare_pass(const StepArgs<R> &a, const FFParams &p)
+{
+  __shared__ double sx[(BLOCK + 2) * 9];
+  PrepareTile<R, BLOCK> t;
+  for (int r0 = blockIdx.x * BLOCK; r0 < a.n_run; r0 += gridDim.x * BLOCK) {
+    t.compute(a, p, r0, sx);
+    t.store(a, r0);
+  }
+  t.reduce(a.nl);
+}
 
 // Pair-list rebuild decision.  A residue pair is needed when one of its
 // tested bead pairs is inside that term's cutoff; in contact-bead distance
@@ -360,52 +387,84 @@ template <typename R> __global__ void k_prepare(StepArgs<R> a, FFParams p) { pre
 // complete while R_need(t) + 2 * max displacement <= radius.
 __device__ __forceinline__ void nl_decide(NLState *nl, int force, long long *step)
 {
-  if (step) (*step)++;
   NLState &s = *nl;
-  float need = fmaxf(fmaxf(s.r_contact, s.r_dssp + s.bO + s.bN), fmaxf(s.r_pap + 2.f * s.bCA, s.r_ev + 2.f * s.bAll));
+  // everything read before anything is written: the loads are in flight together
+  const float bO = s.bO, bN = s.bN, bCA = s.bCA, bAll = s.bAll, bCBx = s.bCBx, bOx = s.bOx, bNCA = s.bNCA;
+  const float d2max = s.d2max, ld2 = s.lst_d2max, pair_cut = s.lst_pair_cut, r_list = s.r_list, skin = s.skin;
+  const float r_contact = s.r_contact, r_dssp = s.r_dssp, r_pap = s.r_pap, r_ev = s.r_ev;
+  const int every = s.every, since = s.steps_since, nbuilds = s.nbuilds, lst_force = s.lst_force;
+  const long long st = step ? *step : 0;
+  float cutk[18];
+#pragma unroll
+  for (int k = 0; k < 18; k++) cutk[k] = (&s.ev_cutk[0][0][0])[k];
+  float need = fmaxf(fmaxf(r_contact, r_dssp + bO + bN), fmaxf(r_pap + 2.f * bCA, r_ev + 2.f * bAll));
   // residue pairs whose CAs were within the half list's reach at the last
   // emulated build: their contact beads are at most that reach + twice the
   // CA displacement since then + twice the CA-to-contact-bead offset apart
-  if (s.lst_pair_cut > 0.f) need = fmaxf(need, s.lst_pair_cut + 2.f * sqrtf(s.lst_d2max) + 2.f * s.bCA + 0.01f);
-  float disp = sqrtf(s.d2max);
-  bool rb = force || s.r_list <= 0.f || need + 2.f * disp > s.r_list || (s.every > 0 && s.steps_since + 1 >= s.every);
-  if (rb) {
-    s.npairs = 0;  // k_nl_build appends
-    s.r_list = need + s.skin;
-    s.steps_since = 0;
-    s.nbuilds++;
-  } else {
-    s.steps_since++;
-  }
-  s.rebuild = rb;
-  s.need = need;
-  s.fm_next = 0;
-  s.bCAx = fmaxf(s.bCBx, s.bOx);
+  if (pair_cut > 0.f) need = fmaxf(need, pair_cut + 2.f * sqrtf(ld2) + 2.f * bCA + 0.01f);
+  const float disp = sqrtf(d2max);
+  const bool rb = force || r_list <= 0.f || need + 2.f * disp > r_list || (every > 0 && since + 1 >= every);
   // |b(i) - b'(j)| >= |CA(i) - CA(j)| - reach(b) - reach(b'): two residues
   // whose CAs are farther apart than the largest cutoff + reaches of any
   // interacting bead kinds have no bead pair in excluded-volume range
   // (0.01 A covers rounding)
-  s.ev_reach[0] = 0.f;
-  s.ev_reach[1] = s.bCBx;
-  s.ev_reach[2] = s.bOx;
+  const float reach[3] = {0.f, bCBx, bOx};
   float pre = 0.f;
-  for (int r = 0; r < 2; r++)
-    for (int b0 = 0; b0 < 3; b0++)
-      for (int b1 = 0; b1 < 3; b1++)
-        if (s.ev_cutk[r][b0][b1] > 0.f) pre = fmaxf(pre, s.ev_cutk[r][b0][b1] + s.ev_reach[b0] + s.ev_reach[b1]);
+#pragma unroll
+  for (int k = 0; k < 18; k++)
+    if (cutk[k] > 0.f) pre = fmaxf(pre, cutk[k] + reach[k % 9 / 3] + reach[k % 3]);
   pre += 0.01f;
-  s.ev_pre_sq = pre * pre;
   // |O(i) - N(j)| >= |CA(i) - CA(j)| - |O(i) - CA(i)| - |N(j) - CA(j)|, and bCAx bounds |O - CA|
-  const float dpre = s.r_dssp + s.bCAx + s.bNCA + 0.01f;
+  const float bCAx = fmaxf(bCBx, bOx), dpre = r_dssp + bCAx + bNCA + 0.01f;
+  if (step) *step = st + 1;
+  if (rb) {
+    s.npairs = 0;  // k_nl_build appends
+    s.r_list = need + skin;
+    s.nbuilds = nbuilds + 1;
+  }
+  s.steps_since = rb ? 0 : since + 1;
+  s.rebuild = rb;
+  s.need = need;
+  s.fm_next = 0;
+  s.bCAx = bCAx;
+  s.ev_reach[0] = 0.f;
+  s.ev_reach[1] = bCBx;
+  s.ev_reach[2] = bOx;
+  s.ev_pre_sq = pre * pre;
   s.dssp_pre_sq = dpre * dpre;
   s.d2max = s.bO = s.bN = s.bCA = s.bAll = s.bCBx = s.bOx = s.bNCA = 0.f;
   s.n_dssp = s.n_pap = 0;
-  s.lst_setup = s.lst_force;
+  s.lst_setup = lst_force;
   s.lst_force = 0;
   s.lst_d2max = 0.f;
 }
 
-__global__ void k_nl_decide(NLState *nl, int force, long long *step) { nl_decide(nl, force, step); }
+// A block per kPrepBlock residues.  The last block whose maxima have arrived
+// takes the decision: its thread sees every block's (a block's are ordered
+// before its arrival by the first warp's fence, and the fence after the last
+// arrival orders the reads).  The maxima go out before the stores, which the
+// fence would otherwise wait for.  As a kernel of its own for one thread the
+// decision was 3.5 us of every step; with strided 8-byte accesses and an FP64
+// root per quantity and thread this one took 43 us on 283,000 residues (133 MB).
+constexpr int kPrepBlock = 128;
+template <typename R> __global__ void __launch_bounds__(kPrepBlock) k_prepare(StepArgs<R> a, FFParams p, int force, long long *step)
+{
+  __shared__ double sx[(kPrepBlock + 2) * 9];
+  const int r0 = blockIdx.x * kPrepBlock;
+  PrepareTile<R, kPrepBlock> t;
+  t.compute(a, p, r0, sx);
+  t.reduce(a.nl);
+  if (threadIdx.x < 32) {
+    __threadfence();
+    __syncwarp();
+    if (threadIdx.x == 0 && atomicAdd(&a.nl->prepared, 1) == (int) gridDim.x - 1) {
+      a.nl->prepared = 0;
+      __threadfence();
+      nl_decide(a.nl, force, step);
+    }
+  }
+  t.store(a, r0);
+}
 
 // contact bead of residue r (one load, no dependence on the residue's flags)
 template <typename R> __device__ __forceinline__ V3<double> contact(const DevSys<R> &s, int r)
@@ -438,14 +497,25 @@ struct GridArgs {
   int *sorted;          // [n_res] residues of each gridded replica, by cell, at the replica's residue range
 };
 
-// one block per gridded replica: bounding box, grid shape, cleared counts
-template <typename R> __global__ void k_grid_setup(StepArgs<R> a, GridArgs g)
+__device__ __forceinline__ int grid_coord(float p, float o, float inv, int n)
+{
+  return min(n - 1, max(0, (int) ((p - o) * inv)));
+}
+
+// One block of 1,024 threads per gridded replica, on the steps that rebuild:
+// bounding box and grid shape, each residue's cell and the cell counts, cell
+// starts (exclusive scan, offset by the replica's first residue; a run of
+// cells a thread), and the residues placed in their cells.  Four kernels for
+// this cost their launches on every step, about 2 us each, and the scan 1,024
+// cells at a time some 100 us of a rebuild on 40,000 residues.
+constexpr int kGridThreads = 1024;
+template <typename R> __global__ void __launch_bounds__(kGridThreads) k_grid_build(StepArgs<R> a, GridArgs g)
 {
   if (!a.nl->rebuild) return;
-  const int b = blockIdx.x, rep = g.big_rep[b];
+  const int b = blockIdx.x, rep = g.big_rep[b], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r0 = a.sys_begin[rep], r1 = a.sys_end[rep];
   float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
-  for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+  for (int r = r0 + tid; r < r1; r += kGridThreads) {
     const V3<double> c = contact(a.s, r);
     const float p[3] = {(float) c.x, (float) c.y, (float) c.z};
     for (int k = 0; k < 3; k++) {
@@ -454,21 +524,22 @@ template <typename R> __global__ void k_grid_setup(StepArgs<R> a, GridArgs g)
     }
   }
   __shared__ float sl[3][32], sh[3][32];
+  __shared__ GridDesc sd;
   for (int k = 0; k < 3; k++) {
     for (int o = 16; o > 0; o >>= 1) {
       lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
       hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
     }
-    if ((threadIdx.x & 31) == 0) {
-      sl[k][threadIdx.x >> 5] = lo[k];
-      sh[k][threadIdx.x >> 5] = hi[k];
+    if (lane == 0) {
+      sl[k][warp] = lo[k];
+      sh[k][warp] = hi[k];
     }
   }
   __syncthreads();
-  GridDesc &d = g.desc[b];
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
+    GridDesc d = g.desc[b];
     for (int k = 0; k < 3; k++)
-      for (int w = 1; w < (int) (blockDim.x >> 5); w++) {
+      for (int w = 1; w < 32; w++) {
         sl[k][0] = fminf(sl[k][0], sl[k][w]);
         sh[k][0] = fmaxf(sh[k][0], sh[k][w]);
       }
@@ -491,80 +562,58 @@ template <typename R> __global__ void k_grid_setup(StepArgs<R> a, GridArgs g)
     d.nx = n[0];
     d.ny = n[1];
     d.nz = n[2];
+    g.desc[b] = d;
+    sd = d;
   }
   __syncthreads();
-  for (int c = threadIdx.x; c < d.cap; c += blockDim.x) {
-    g.cell_count[d.cell0 + c] = 0;
-    g.cell_fill[d.cell0 + c] = 0;
-  }
-}
-
-__device__ __forceinline__ int grid_coord(float p, float o, float inv, int n)
-{
-  return min(n - 1, max(0, (int) ((p - o) * inv)));
-}
-
-// thread per residue of a gridded replica: its cell, and the cell counts
-template <typename R> __global__ void k_grid_count(StepArgs<R> a, GridArgs g)
-{
-  if (!a.nl->rebuild) return;
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= a.s.n_res || a.res_sys[r] < 0) return;
-  const int b = g.big_of[a.res_sys[r]];
-  if (b < 0) return;
-  const GridDesc d = g.desc[b];
-  const V3<double> c = contact(a.s, r);
-  const int cx = grid_coord((float) c.x, d.ox, d.inv_cell, d.nx), cy = grid_coord((float) c.y, d.oy, d.inv_cell, d.ny),
-            cz = grid_coord((float) c.z, d.oz, d.inv_cell, d.nz);
-  const int cell = d.cell0 + (cz * d.ny + cy) * d.nx + cx;
-  g.res_cell[r] = cell;
-  atomicAdd(&g.cell_count[cell], 1);
-}
-
-// one block per gridded replica: cell starts (exclusive scan, offset by the
-// replica's first residue) in chunks of blockDim.x cells
-template <typename R> __global__ void k_grid_scan(StepArgs<R> a, GridArgs g)
-{
-  if (!a.nl->rebuild) return;
-  const int b = blockIdx.x;
-  const GridDesc d = g.desc[b];
-  const int ncell = d.nx * d.ny * d.nz;
-  __shared__ int part[1024];
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = a.sys_begin[g.big_rep[b]];
+  const GridDesc d = sd;
+  const int ncell = d.nx * d.ny * d.nz;  // at most cap
+  for (int c = tid; c < ncell; c += kGridThreads) g.cell_count[d.cell0 + c] = 0;
   __syncthreads();
-  for (int c0 = 0; c0 < ncell; c0 += blockDim.x) {
-    const int c = c0 + threadIdx.x;
-    const int v = c < ncell ? g.cell_count[d.cell0 + c] : 0;
-    part[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < (int) blockDim.x; o <<= 1) {  // inclusive Hillis-Steele scan
-      const int add = threadIdx.x >= (unsigned) o ? part[threadIdx.x - o] : 0;
-      __syncthreads();
-      part[threadIdx.x] += add;
-      __syncthreads();
+  for (int r = r0 + tid; r < r1; r += kGridThreads) {
+    const V3<double> c = contact(a.s, r);
+    const int cx = grid_coord((float) c.x, d.ox, d.inv_cell, d.nx), cy = grid_coord((float) c.y, d.oy, d.inv_cell, d.ny),
+              cz = grid_coord((float) c.z, d.oz, d.inv_cell, d.nz);
+    const int cell = d.cell0 + (cz * d.ny + cy) * d.nx + cx;
+    g.res_cell[r] = cell;
+    atomicAdd(&g.cell_count[cell], 1);
+  }
+  __syncthreads();
+  // thread t's run of cells
+  const int run = (ncell + kGridThreads - 1) / kGridThreads, c0 = min(ncell, tid * run), c1 = min(ncell, c0 + run);
+  int sum = 0;
+  for (int c = c0; c < c1; c++) sum += __ldcg(&g.cell_count[d.cell0 + c]);
+  int inc = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  __shared__ int wsum[32];
+  if (lane == 31) wsum[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    int v = wsum[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += t;
     }
-    if (c < ncell) g.cell_start[d.cell0 + c] = carry + part[threadIdx.x] - v;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry += part[threadIdx.x];
-    __syncthreads();
+    wsum[lane] = v;
   }
-}
-
-// thread per residue of a gridded replica: place it in its cell's range
-template <typename R> __global__ void k_grid_fill(StepArgs<R> a, GridArgs g)
-{
-  if (!a.nl->rebuild) return;
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= a.s.n_res || a.res_sys[r] < 0 || g.big_of[a.res_sys[r]] < 0) return;
-  const int cell = g.res_cell[r];
-  g.sorted[g.cell_start[cell] + atomicAdd(&g.cell_fill[cell], 1)] = r;
+  __syncthreads();
+  int at = r0 + inc - sum + (warp ? wsum[warp - 1] : 0);
+  for (int c = c0; c < c1; c++) {
+    g.cell_start[d.cell0 + c] = at;
+    g.cell_fill[d.cell0 + c] = at;
+    at += __ldcg(&g.cell_count[d.cell0 + c]);
+  }
+  __syncthreads();
+  for (int r = r0 + tid; r < r1; r += kGridThreads) g.sorted[atomicAdd(&g.cell_fill[g.res_cell[r]], 1)] = r;
 }
 
 // Residue pair list: every pair i < j of one replica whose contact beads are
 // closer than r_list, as (i, j) in a flat array.  One warp per residue scans
-// the candidates twice (count, then write after one atomic reservation), so
-// a residue's pairs are contiguous.  Candidates: the higher residues of its
+// the candidates (count, then write after one atomic reservation), so a
+// residue's pairs are contiguous.  Candidates: the higher residues of its
 // replica, or for a gridded replica the residues of the 27 cells around its
 // own.  Every pair pass below runs one thread per listed (or near) pair and
 // scatters to both residues with fixed-point atomics: each pair is evaluated
@@ -591,12 +640,11 @@ template <typename R> __device__ __forceinline__ void nl_build_one(const StepArg
     cy = (cell / d.nx) % d.ny;
     cz = cell / (d.nx * d.ny);
   }
-  auto scan = [&](auto &&visit) {  // visit(j, take) for every candidate, warp-uniform trip counts
+  // visit(it, j, in): every group of 32 candidates, warp-uniform trip counts
+  auto scan = [&](auto &&visit) {
+    int it = 0;
     if (b < 0) {
-      for (int j0 = i + 1; j0 < sys_end; j0 += 32) {
-        const int j = j0 + lane;
-        visit(j, j < sys_end && norm2(diff<R>(ci, contact(s, j))) < rl2);
-      }
+      for (int j0 = i + 1; j0 < sys_end; j0 += 32) visit(it++, j0 + lane, j0 + lane < sys_end);
       return;
     }
     for (int z = max(0, cz - 1); z <= min(d.nz - 1, cz + 1); z++)
@@ -607,12 +655,20 @@ template <typename R> __device__ __forceinline__ void nl_build_one(const StepArg
           for (int kb = k0; kb < k1; kb += 32) {
             const int k = kb + lane;
             const int j = k < k1 ? g.sorted[k] : -1;
-            visit(j, j > i && norm2(diff<R>(ci, contact(s, j))) < rl2);
+            visit(it++, j, j > i);
           }
         }
   };
+  auto close = [&](int j, bool in) { return in && norm2(diff<R>(ci, contact(s, j))) < rl2; };
+  // The first scan counts; it keeps each group's verdicts (lane t those of
+  // groups t and t + 32), so that the second only writes.
   int count = 0;
-  scan([&](int, bool take) { count += __popc(__ballot_sync(0xffffffffu, take)); });
+  unsigned kept[2] = {0u, 0u};
+  scan([&](int it, int j, bool in) {
+    const unsigned m = __ballot_sync(0xffffffffu, close(j, in));
+    count += __popc(m);
+    if ((it & 31) == lane) kept[0] = it < 32 ? m : kept[0], kept[1] = it >= 32 && it < 64 ? m : kept[1];
+  });
   int base = 0;
   if (lane == 0 && count) base = atomicAdd(&a.nl->npairs, count);
   base = __shfl_sync(0xffffffffu, base, 0);
@@ -623,10 +679,11 @@ template <typename R> __device__ __forceinline__ void nl_build_one(const StepArg
   }
   int at = base;
   if (count)
-    scan([&](int j, bool take) {
-      const unsigned m = __ballot_sync(0xffffffffu, take);
+    scan([&](int it, int j, bool in) {
+      const unsigned m = it < 64 ? __shfl_sync(0xffffffffu, it < 32 ? kept[0] : kept[1], it & 31)
+                                 : __ballot_sync(0xffffffffu, close(j, in));
       const int k = at + __popc(m & ((1u << lane) - 1u));
-      if (take && k < a.pcap) a.pairs[k] = make_int2(i, j);
+      if ((m >> lane & 1u) && k < a.pcap) a.pairs[k] = make_int2(i, j);
       at += __popc(m);
     });
 }

@@ -191,7 +191,7 @@ template <typename R> __global__ void __launch_bounds__(kStepThreads, 2) k_step(
   unsigned kbase = 0;
 
   const Span all{(int) (blockIdx.x * kStepThreads + threadIdx.x), (int) (gridDim.x * kStepThreads)};
-  prepare_pass(a, p, all);
+  prepare_pass<R, kStepThreads>(a, p);
   bool ok = grid_sync(b, 0, seen[0], 0, kStepThreads, true, q.bar_wait_limit, q.hold, FirstSerial{a.nl, a.step, b});
   if ((int) threadIdx.x >= pass_threads) {
     if (ok) fragmem_take_units(a, p, q, ring, wsm, kbase);
