@@ -68,6 +68,31 @@ template <typename T> struct DBuf {
   }
 };
 
+// Page-locked host memory: copies from and to it are queued, where a copy of
+// pageable memory holds the calling thread.  Kept by the handle, grown when
+// asked for more (nothing may be in flight on it then).
+struct PinnedBuf {
+  char *p = nullptr;
+  size_t n = 0;
+  PinnedBuf() = default;
+  PinnedBuf(const PinnedBuf &) = delete;
+  PinnedBuf &operator=(const PinnedBuf &) = delete;
+  ~PinnedBuf()
+  {
+    if (p) cudaFreeHost(p);
+  }
+  void need(size_t bytes)
+  {
+    if (bytes <= n) return;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    n = 0;
+    CK(cudaHostAlloc((void **) &p, bytes, cudaHostAllocDefault));
+    n = bytes;
+  }
+  template <typename T> T *at(size_t byte) const { return reinterpret_cast<T *>(p + byte); }
+};
+
 constexpr double FTM2V = 1.0 / 48.88821291 / 48.88821291;
 constexpr double MVV2E = 48.88821291 * 48.88821291;
 constexpr double BOLTZ = 0.0019872067;
@@ -219,7 +244,13 @@ template <typename R> class Engine : public EngineBase {
   int groups_all = dev::G_FIX | dev::G_PAIR | dev::G_BOND;
   double skin = 2.0;
   int neigh_every = 0;
-  std::vector<double> hx, hv;  // host staging (internal order)
+  // Host staging of the calls' small inputs and results (run parameters, list
+  // state, energies) and, on single-system handles, of awsem_compute's arrays.
+  // Every call that queues copies on it synchronises s0 before it returns.
+  PinnedBuf h_call, h_io;
+  // h_call: list state, energies, integrator, step counter, then per replica its run window and seed
+  static constexpr size_t kHostEnergy = (sizeof(dev::NLState) + 63) / 64 * 64, kHostInteg = kHostEnergy + 8 * E_SLOTS,
+                          kHostStep = (kHostInteg + sizeof(dev::Integrator) + 7) / 8 * 8, kHostRuns = kHostStep + 16;
 
   ~Engine() override
   {
@@ -572,6 +603,7 @@ template <typename R> class Engine : public EngineBase {
     CK(cudaMemcpyAsync(nl.p, &st, sizeof st, cudaMemcpyHostToDevice, s0));
     long long s = step;
     CK(cudaMemcpyAsync(dstep.p, &s, sizeof s, cudaMemcpyHostToDevice, s0));
+    h_call.need(kHostRuns + (sizeof(dev::SlotRun) + 8) * (size_t) std::max(in.n_sys, 1));
     e_fix.alloc((size_t) efix_slots * nn);
     e_fix.zero(s0);
     dacc.alloc((size_t) 3 * nn);
@@ -580,7 +612,10 @@ template <typename R> class Engine : public EngineBase {
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     sms_ = sms;
     hb_blocks = std::max(1, std::min((nn * 8 + 127) / 128, 16 * sms));
-    if (!server_pending) setup_grids();
+    if (!server_pending) {
+      setup_grids();
+      setup_transfer();
+    }
     // size the pair list from a first build: room for 4x the initial pairs
     // (chains that collapse gain neighbours), at least pairs_per_res per residue
     resize_pairs(std::max<long long>(64, 16LL * nn));
@@ -798,50 +833,88 @@ template <typename R> class Engine : public EngineBase {
     if (n_sys() != 1) throw std::invalid_argument(std::string(what) + " needs a single-system handle");
   }
 
+  // An evaluation is a fixed sequence on fixed buffers -- positions from the
+  // page-locked staging, forces, energies and the list state back to it -- so
+  // that a handle's third call with the same term groups records it in a graph
+  // and later calls launch that (one launch instead of some twenty; the first
+  // two, for programs that need a single evaluation, do not pay for the
+  // recording).  The host waits once, at the end.
+  cudaGraphExec_t eval_graph = nullptr;
+  int eval_groups = -1, eval_calls = 0;
+
+  void queue_evaluation(int groups)
+  {
+    const int na = natoms(), tb = 256, nb = (na + tb - 1) / tb;
+    const size_t bytes = sizeof(double) * 3 * na;
+    CK(cudaMemcpyAsync(stage.p, h_io.p, bytes, cudaMemcpyHostToDevice, s0));
+    CK(cudaMemcpyAsync(dstep.p, h_call.at<long long>(kHostStep), sizeof(long long), cudaMemcpyHostToDevice, s0));
+    dev::k_gather3<<<nb, tb, 0, s0>>>(stage.p, perm.p, na, x.p);
+    zero_unwritten_energies(groups);
+    auto a = args(groups);
+    launch_eval(a, false);
+    if (lists_emulated()) dev::k_list_hold<R><<<(n_run() + 127) / 128, 128, 0, s0>>>(a);
+    dev::k_total_force<R><<<nb, tb, 0, s0>>>(a, ftot.p, perm.p, stage.p);
+    reduce_energies();
+    CK(cudaMemcpyAsync(h_io.p + bytes, stage.p, bytes, cudaMemcpyDeviceToHost, s0));
+    CK(cudaMemcpyAsync(h_call.p + kHostEnergy, energy.p, sizeof(double) * E_SLOTS, cudaMemcpyDeviceToHost, s0));
+    CK(cudaMemcpyAsync(h_call.p, nl.p, sizeof(dev::NLState), cudaMemcpyDeviceToHost, s0));
+  }
+
   void compute(long long st, const double *x_ext, double *f_ext, double *energies_out, int groups) override
   {
     need_single("awsem_compute");
+    if (server) throw std::invalid_argument("awsem_compute: not available on a serving handle");
     cont_step = -1;
-    const std::vector<int> &ext = in.ext_of[0];
-    int na = natoms();
-    hx.resize((size_t) 3 * na);
-    for (int a = 0; a < na; a++)
-      for (int k = 0; k < 3; k++) hx[3 * a + k] = x_ext[3 * ext[a] + k];
-    CK(cudaMemcpyAsync(x.p, hx.data(), sizeof(double) * 3 * na, cudaMemcpyHostToDevice, s0));
-    CK(cudaMemcpyAsync(dstep.p, &st, sizeof st, cudaMemcpyHostToDevice, s0));
+    const int na = natoms();
+    const size_t bytes = sizeof(double) * 3 * na;
+    h_io.need(2 * bytes);
+    std::memcpy(h_io.p, x_ext, bytes);
+    *h_call.at<long long>(kHostStep) = st;
     step = st;
-    zero_unwritten_energies(groups);
     if (lists_emulated()) {
       // the host's MD loop decides whether this evaluation's lists are new
       set_list_flags(next_compute_built, 1);
       next_compute_built = 1;
     }
-    int tb = 256;
+    if (groups != eval_groups) {
+      release_eval_graph();
+      eval_groups = groups;
+    }
+    eval_calls++;
+    if (eval_calls >= 3 && !eval_graph && !sel_cap) {
+      cudaGraph_t graph;
+      CK(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
+      queue_evaluation(groups);
+      CK(cudaStreamEndCapture(s0, &graph));
+      set_node_priorities(graph);
+      CK(cudaGraphInstantiate(&eval_graph, graph, 0));
+      CK(cudaGraphDestroy(graph));
+    }
     for (int attempt = 0; attempt < 2; attempt++) {
-      auto a = args(groups);
-      launch_eval(a, false);
-      if (lists_emulated()) dev::k_list_hold<R><<<(n_run() + 127) / 128, 128, 0, s0>>>(a);
-      dev::k_total_force<R><<<(3 * na + tb - 1) / tb, tb, 0, s0>>>(a, ftot.p);
-      reduce_energies();
+      if (eval_graph && !sel_cap)
+        CK(cudaGraphLaunch(eval_graph, s0));
+      else
+        queue_evaluation(groups);
       CK(cudaGetLastError());
+      CK(cudaStreamSynchronize(s0));
       // an evaluation whose pair list overflowed runs again on a grown list
       // (it changes no state, unless LAMMPS's lists are emulated, whose
       // per-step bookkeeping it advances: then the overflow is reported)
-      int ovf = 0;
-      CK(cudaMemcpyAsync(&ovf, &nl.p->overflow, sizeof ovf, cudaMemcpyDeviceToHost, s0));
-      CK(cudaStreamSynchronize(s0));
+      const int ovf = h_call.at<dev::NLState>(0)->overflow;
       if (!ovf || attempt == 1 || lists_emulated()) break;
       grow_pairs(ovf);
     }
-    std::vector<double> f((size_t) 3 * na);
-    CK(cudaMemcpyAsync(f.data(), ftot.p, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, s0));
-    double e[E_SLOTS];
-    CK(cudaMemcpyAsync(e, energy.p, sizeof e, cudaMemcpyDeviceToHost, s0));
-    CK(cudaStreamSynchronize(s0));
-    check_list();
-    for (int at = 0; at < na; at++)
-      for (int k = 0; k < 3; k++) f_ext[3 * ext[at] + k] += f[3 * at + k];
-    if (energies_out) finish_energies(e, energies_out, false);
+    check_state(*h_call.at<dev::NLState>(0));
+    const double *f = reinterpret_cast<const double *>(h_io.p + bytes);
+    for (int k = 0; k < 3 * na; k++) f_ext[k] += f[k];
+    if (energies_out) finish_energies(h_call.at<double>(kHostEnergy), energies_out, false);
+  }
+
+  void release_eval_graph()
+  {
+    if (eval_graph) cudaGraphExecDestroy(eval_graph);
+    eval_graph = nullptr;
+    eval_calls = 0;
   }
 
   void finish_energies(const double *e, double *out, bool with_ke)
@@ -877,8 +950,14 @@ template <typename R> class Engine : public EngineBase {
 
   void check_list()
   {
-    dev::NLState st;
-    CK(cudaMemcpy(&st, nl.p, sizeof st, cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(h_call.p, nl.p, sizeof(dev::NLState), cudaMemcpyDeviceToHost, s0));
+    CK(cudaStreamSynchronize(s0));
+    check_state(*h_call.at<dev::NLState>(0));
+  }
+
+  // errors an evaluation flagged in its list state (a copy of it, taken after the evaluation)
+  void check_state(const dev::NLState &st)
+  {
     if (st.bad_x) {
       // positions are inputs: the next call with finite ones is clean
       set_nl_field(&dev::NLState::bad_x, 0);
@@ -917,54 +996,70 @@ template <typename R> class Engine : public EngineBase {
     if (rep < 0 || rep >= n_sys()) throw std::invalid_argument("replica index out of range");
   }
 
-  // Whole-batch state transfer: one copy each way through a device staging
-  // buffer, and a gather/scatter kernel between caller order and internal order.
+  // State transfer: a copy per array each way through a device staging buffer,
+  // and a gather/scatter kernel between caller order and internal order.
   DBuf<int> perm;              // internal atom -> position in the concatenated caller arrays
-  DBuf<double> stage;          // [n_atoms][3]
+  DBuf<double> stage;          // [2][n_atoms][3]: positions, velocities
 
-  void ensure_perm()
+  void setup_transfer()
   {
-    if (perm.p) return;
-    if (server) throw std::invalid_argument("whole-batch state transfer is not available on a serving handle");
     std::vector<int> pm(natoms());
     for (int r = 0; r < n_sys(); r++) {
       const int a0 = rep_atom0(r), na = rep_atoms(r);
       for (int a = 0; a < na; a++) pm[a0 + a] = a0 + in.ext_of[r][a];
     }
     perm.upload(pm, s0);
-    stage.alloc((size_t) 3 * natoms());
+    stage.alloc((size_t) 6 * natoms());
+    CK(cudaStreamSynchronize(s0));  // pm goes out of scope
   }
 
-  void set_state_all(const double *x_ext, const double *v_ext) override
+  // atoms [a0, a0 + na) from / to the caller's arrays of those atoms (either may be null)
+  void put_atoms(int a0, int na, const double *x_ext, const double *v_ext)
   {
-    ensure_perm();
+    if (server) throw std::invalid_argument("whole-batch state transfer is not available on a serving handle");
     cont_step = -1;
-    const int na = natoms(), tb = 256;
+    const int tb = 256;
     for (int k = 0; k < 2; k++) {
       const double *src = k ? v_ext : x_ext;
-      if (!src) continue;
-      CK(cudaMemcpyAsync(stage.p, src, sizeof(double) * 3 * na, cudaMemcpyHostToDevice, s0));
-      dev::k_gather3<<<(na + tb - 1) / tb, tb, 0, s0>>>(stage.p, perm.p, na, k ? v.p : x.p);
+      if (!src || !na) continue;
+      double *st = stage.p + (size_t) 3 * natoms() * k;
+      CK(cudaMemcpyAsync(st + (size_t) 3 * a0, src, sizeof(double) * 3 * na, cudaMemcpyHostToDevice, s0));
+      dev::k_gather3<<<(na + tb - 1) / tb, tb, 0, s0>>>(st, perm.p + a0, na, (k ? v.p : x.p) + (size_t) 3 * a0);
     }
     CK(cudaStreamSynchronize(s0));
   }
+  void get_atoms(int a0, int na, const double *from[2], double *to[2])
+  {
+    if (server) throw std::invalid_argument("whole-batch state transfer is not available on a serving handle");
+    const int tb = 256;
+    for (int k = 0; k < 2; k++) {
+      if (!to[k] || !na) continue;
+      double *st = stage.p + (size_t) 3 * natoms() * k;
+      dev::k_scatter3<<<(na + tb - 1) / tb, tb, 0, s0>>>(from[k] + (size_t) 3 * a0, perm.p + a0, na, st);
+    }
+    for (int k = 0; k < 2; k++)
+      if (to[k] && na)
+        CK(cudaMemcpyAsync(to[k], stage.p + (size_t) 3 * (natoms() * (size_t) k + a0), sizeof(double) * 3 * na,
+                           cudaMemcpyDeviceToHost, s0));
+    CK(cudaStreamSynchronize(s0));
+  }
+
+  void set_state_all(const double *x_ext, const double *v_ext) override { put_atoms(0, natoms(), x_ext, v_ext); }
 
   void get_state_all(double *x_ext, double *v_ext) override
   {
-    ensure_perm();
-    const int na = natoms(), tb = 256;
-    for (int k = 0; k < 2; k++) {
-      double *dst = k ? v_ext : x_ext;
-      if (!dst) continue;
-      dev::k_scatter3<<<(na + tb - 1) / tb, tb, 0, s0>>>(k ? v.p : x.p, perm.p, na, stage.p);
-      CK(cudaMemcpyAsync(dst, stage.p, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, s0));
-      CK(cudaStreamSynchronize(s0));
-    }
+    const double *from[2] = {x.p, v.p};
+    double *to[2] = {x_ext, v_ext};
+    get_atoms(0, natoms(), from, to);
   }
 
   void set_state(int rep, const double *x_ext, const double *v_ext) override
   {
     check_rep(rep);
+    if (!server) {
+      put_atoms(rep_atom0(rep), rep_atoms(rep), x_ext, v_ext);
+      return;
+    }
     cont_step = -1;
     const std::vector<int> &ext = in.ext_of[rep];
     int a0 = rep_atom0(rep), na = rep_atoms(rep);
@@ -979,27 +1074,42 @@ template <typename R> class Engine : public EngineBase {
     CK(cudaStreamSynchronize(s0));
   }
 
+  // a replica's atoms from two device arrays to the caller's (either may be null); a serving handle's requests come
+  // and go, so their order stays on the host
+  void get_replica(int rep, const double *from0, const double *from1, double *to0, double *to1)
+  {
+    const int a0 = rep_atom0(rep), na = rep_atoms(rep);
+    const double *from[2] = {from0, from1};
+    double *to[2] = {to0, to1};
+    if (!server) {
+      get_atoms(a0, na, from, to);
+      return;
+    }
+    const std::vector<int> &ext = in.ext_of[rep];
+    const size_t bytes = sizeof(double) * 3 * na;
+    h_io.need(2 * bytes);
+    for (int k = 0; k < 2; k++)
+      if (to[k]) CK(cudaMemcpyAsync(h_io.p + k * bytes, from[k] + 3 * (size_t) a0, bytes, cudaMemcpyDeviceToHost, s0));
+    CK(cudaStreamSynchronize(s0));
+    for (int k = 0; k < 2; k++) {
+      if (!to[k]) continue;
+      const double *h = reinterpret_cast<const double *>(h_io.p + k * bytes);
+      for (int a = 0; a < na; a++)
+        for (int c = 0; c < 3; c++) to[k][3 * ext[a] + c] = h[3 * a + c];
+    }
+  }
+
   void get_state(int rep, double *x_ext, double *v_ext) override
   {
     check_rep(rep);
-    const std::vector<int> &ext = in.ext_of[rep];
-    int a0 = rep_atom0(rep), na = rep_atoms(rep);
-    std::vector<double> hx2((size_t) 3 * na), hv2((size_t) 3 * na);
-    CK(cudaMemcpyAsync(hx2.data(), x.p + 3 * (size_t) a0, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, s0));
-    CK(cudaMemcpyAsync(hv2.data(), v.p + 3 * (size_t) a0, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, s0));
-    CK(cudaStreamSynchronize(s0));
-    for (int a = 0; a < na; a++)
-      for (int k = 0; k < 3; k++) {
-        if (x_ext) x_ext[3 * ext[a] + k] = hx2[3 * a + k];
-        if (v_ext) v_ext[3 * ext[a] + k] = hv2[3 * a + k];
-      }
+    get_replica(rep, x.p, v.p, x_ext, v_ext);
   }
 
   // Graphs of `count` consecutive MD steps.  Every per-run value (integrator
   // parameters, step counter, thermo buffer) lives in device memory, so a
   // graph stays valid across runs and is instantiated once.
-  cudaGraphExec_t graphs[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [thermo][chunk]
-  static constexpr int kChunk = 25;
+  static constexpr int kChunks[3] = {1, 5, 25};  // steps per graph
+  cudaGraphExec_t graphs[2][3] = {};             // [thermo][chunk]
   DBuf<dev::Integrator> d_integ;
   DBuf<dev::SlotRun> slot_run;  // [n_sys] run window of each replica
   long long thermo_nrows = 1;
@@ -1163,8 +1273,23 @@ template <typename R> class Engine : public EngineBase {
     }
   }
 
+  // the steps of a run or an advance, in the longest graphs that fit
+  void launch_steps(long long total, int tv)
+  {
+    for (int c = 2; c >= 0; c--)
+      for (; total >= kChunks[c]; total -= kChunks[c]) CK(cudaGraphLaunch(graphs[tv][c], s0));
+  }
+  void capture_for(long long total, int tv)
+  {
+    for (int c = 2; c >= 0; c--) {
+      if (total >= kChunks[c] && !graphs[tv][c]) capture_steps(graphs[tv][c], kChunks[c], tv != 0);
+      total %= kChunks[c];
+    }
+  }
+
   void release_graphs()
   {
+    release_eval_graph();
     for (auto &row : graphs)
       for (auto &g : row)
         if (g) {
@@ -1549,17 +1674,21 @@ template <typename R> class Engine : public EngineBase {
     const long long rows = cont ? nsteps : nsteps + 1;  // evaluations of this call
     dev::Integrator integ = make_integrator(rp, cont ? step + 1 : step);
     integ.stop = step + nsteps;
-    upload_integrator(integ);
-    std::vector<dev::SlotRun> w(n_sys(), dev::SlotRun{wbegin, wend, 0, rp.t_start, rp.t_stop});
-    CK(cudaMemcpyAsync(slot_run.p, w.data(), sizeof(dev::SlotRun) * w.size(), cudaMemcpyHostToDevice, s0));
-    // Langevin seed of each replica: its own when set, else the run's
-    std::vector<unsigned long long> sd(n_sys());
-    for (int k = 0; k < n_sys(); k++) sd[k] = seeds[k] ? seeds[k] : rp.seed;
-    CK(cudaMemcpyAsync(sys_seed.p, sd.data(), sizeof(unsigned long long) * sd.size(), cudaMemcpyHostToDevice, s0));
+    if (!d_integ.p) d_integ.alloc(1);
+    const size_t ns = (size_t) n_sys();
+    *h_call.at<dev::Integrator>(kHostInteg) = integ;
     // a setup evaluation advances the counter to `step`; a continuation starts from it
-    long long pre = cont ? step : step - 1;
-    CK(cudaMemcpyAsync(dstep.p, &pre, sizeof pre, cudaMemcpyHostToDevice, s0));
-    CK(cudaStreamSynchronize(s0));
+    *h_call.at<long long>(kHostStep) = cont ? step : step - 1;
+    dev::SlotRun *const w = h_call.at<dev::SlotRun>(kHostRuns);
+    unsigned long long *const sd = reinterpret_cast<unsigned long long *>(w + ns);
+    for (size_t k = 0; k < ns; k++) {
+      w[k] = dev::SlotRun{wbegin, wend, 0, rp.t_start, rp.t_stop};
+      sd[k] = seeds[k] ? seeds[k] : rp.seed;  // Langevin seed of each replica: its own when set, else the run's
+    }
+    CK(cudaMemcpyAsync(d_integ.p, h_call.p + kHostInteg, sizeof integ, cudaMemcpyHostToDevice, s0));
+    CK(cudaMemcpyAsync(dstep.p, h_call.p + kHostStep, sizeof(long long), cudaMemcpyHostToDevice, s0));
+    CK(cudaMemcpyAsync(slot_run.p, w, sizeof(dev::SlotRun) * ns, cudaMemcpyHostToDevice, s0));
+    CK(cudaMemcpyAsync(sys_seed.p, sd, sizeof(unsigned long long) * ns, cudaMemcpyHostToDevice, s0));
     bool want_thermo = thermo != nullptr;
     int tv = want_thermo ? 1 : 0;
     if (want_thermo) {
@@ -1573,34 +1702,26 @@ template <typename R> class Engine : public EngineBase {
         }
     }
     long long total = rows;
-    if (!graphs[tv][0]) capture_steps(graphs[tv][0], 1, want_thermo);
-    if (total >= kChunk && !graphs[tv][1]) capture_steps(graphs[tv][1], kChunk, want_thermo);
+    capture_for(total, tv);
     if (!ev_run0) {
       CK(cudaEventCreate(&ev_run0));
       CK(cudaEventCreate(&ev_run1));
     }
-    long long done = 0;
     CK(cudaEventRecord(ev_run0, s0));
     if (cont) {
       const int tb = 128;
       dev::k_continue<R><<<(n_run() + tb - 1) / tb, tb, 0, s0>>>(args(groups_all), d_integ.p, ftot.p, x.p);
       CK(cudaGetLastError());
     }
-    while (total - done >= kChunk) {
-      CK(cudaGraphLaunch(graphs[tv][1], s0));
-      done += kChunk;
-    }
-    while (done < total) {
-      CK(cudaGraphLaunch(graphs[tv][0], s0));
-      done++;
-    }
+    launch_steps(total, tv);
     CK(cudaEventRecord(ev_run1, s0));
+    CK(cudaMemcpyAsync(h_call.p, nl.p, sizeof(dev::NLState), cudaMemcpyDeviceToHost, s0));
     CK(cudaStreamSynchronize(s0));
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, ev_run0, ev_run1));
     last_run_ms = ms;
     step += nsteps;
-    check_list();
+    check_state(*h_call.at<dev::NLState>(0));
     if (want_thermo)
       CK(cudaMemcpy(thermo, thermo_rows.p, sizeof(double) * 4 * rows * n_sys(), cudaMemcpyDeviceToHost));
     if (step < wend) {
@@ -1622,12 +1743,8 @@ template <typename R> class Engine : public EngineBase {
 
   void set_list_flags(int force, int host)
   {
-    dev::NLState st;
-    CK(cudaMemcpyAsync(&st, nl.p, sizeof st, cudaMemcpyDeviceToHost, s0));
-    CK(cudaStreamSynchronize(s0));
-    st.lst_force = force;
-    st.lst_host = host;
-    CK(cudaMemcpyAsync(nl.p, &st, sizeof st, cudaMemcpyHostToDevice, s0));
+    set_nl_field(&dev::NLState::lst_force, force);
+    set_nl_field(&dev::NLState::lst_host, host);
   }
 
   void set_list_built(int built) override { next_compute_built = built ? 1 : 0; }
@@ -1672,35 +1789,26 @@ template <typename R> class Engine : public EngineBase {
     return v;
   }
 
+  // one field of the list state (a copy of pageable memory: `value` has been read when the call returns)
   template <typename F> void set_nl_field(F dev::NLState::*field, F value)
   {
-    dev::NLState st;
-    CK(cudaMemcpyAsync(&st, nl.p, sizeof st, cudaMemcpyDeviceToHost, s0));
-    CK(cudaStreamSynchronize(s0));
-    st.*field = value;
-    CK(cudaMemcpyAsync(nl.p, &st, sizeof st, cudaMemcpyHostToDevice, s0));
+    CK(cudaMemcpyAsync(&(nl.p->*field), &value, sizeof value, cudaMemcpyHostToDevice, s0));
   }
 
   void energies(int rep, double *out) override
   {
     check_rep(rep);
     reduce_energies(rep, 1);
-    double e[E_SLOTS];
-    CK(cudaMemcpyAsync(e, energy.p + (size_t) rep * E_SLOTS, sizeof e, cudaMemcpyDeviceToHost, s0));
+    CK(cudaMemcpyAsync(h_call.p + kHostEnergy, energy.p + (size_t) rep * E_SLOTS, sizeof(double) * E_SLOTS,
+                       cudaMemcpyDeviceToHost, s0));
     CK(cudaStreamSynchronize(s0));
-    finish_energies(e, out, true);
+    finish_energies(h_call.at<double>(kHostEnergy), out, true);
   }
 
   void forces(int rep, double *f_ext) override
   {
     check_rep(rep);
-    const std::vector<int> &ext = in.ext_of[rep];
-    int a0 = rep_atom0(rep), na = rep_atoms(rep);
-    std::vector<double> f((size_t) 3 * na);
-    CK(cudaMemcpyAsync(f.data(), ftot.p + 3 * (size_t) a0, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, s0));
-    CK(cudaStreamSynchronize(s0));
-    for (int at = 0; at < na; at++)
-      for (int k = 0; k < 3; k++) f_ext[3 * ext[at] + k] = f[3 * at + k];
+    get_replica(rep, ftot.p, nullptr, f_ext, nullptr);
   }
 
   void residue_arrays(int rep, double *out) override
@@ -1785,15 +1893,37 @@ template <typename R> class Engine : public EngineBase {
     }
   }
 
+  // A request's arrays go up through a page-locked buffer, so that an
+  // admission queues its copies and waits once (some thirty small copies of
+  // pageable memory and six waits were 0.2 ms of each); a memory table larger
+  // than a quarter of the buffer is copied from where it is.
+  static constexpr size_t kAdmitBuf = 4 << 20;
+  PinnedBuf h_adm;
+  size_t adm_used = 0;  // bytes of h_adm with copies queued since the last wait
+  void put_wait()
+  {
+    CK(cudaStreamSynchronize(s0));
+    adm_used = 0;
+  }
   template <typename T> void put(DBuf<T> &b, size_t at, const T *src, size_t count)
   {
-    if (count) CK(cudaMemcpyAsync(b.p + at, src, count * sizeof(T), cudaMemcpyHostToDevice, s0));
+    const size_t bytes = count * sizeof(T);
+    if (!bytes) return;
+    const void *from = src;
+    if (bytes <= kAdmitBuf / 4) {
+      h_adm.need(kAdmitBuf);
+      if (adm_used + bytes > kAdmitBuf) put_wait();
+      std::memcpy(h_adm.p + adm_used, src, bytes);
+      from = h_adm.p + adm_used;
+      adm_used += (bytes + 63) / 64 * 64;
+    }
+    CK(cudaMemcpyAsync(b.p + at, from, bytes, cudaMemcpyHostToDevice, s0));
   }
   template <typename T> void fill(DBuf<T> &b, size_t at, size_t count, T value)
   {
     std::vector<T> h(count, value);
     put(b, at, h.data(), count);
-    CK(cudaStreamSynchronize(s0));
+    put_wait();
   }
 
   void server_setup(const SharedForceField &f, long long cap_res, int max_slots, long long cap_records, double dt,
@@ -1886,7 +2016,6 @@ template <typename R> class Engine : public EngineBase {
     }
     put(g1, a0, h1.data(), na);
     put(g2, a0, h2.data(), na);
-    CK(cudaStreamSynchronize(s0));
   }
 
   // A request prepared on the host: its system, the slices of its memory
@@ -2010,7 +2139,6 @@ template <typename R> class Engine : public EngineBase {
       int id = base + t.chain_start[c], a = base + t.chain_start[c], b = base + t.chain_end[c];
       put(chain_start, id, &a, 1);
       put(chain_end, id, &b, 1);
-      CK(cudaStreamSynchronize(s0));  // a and b are reused
     }
     for (int k = 0; k < 12; k++) put(aps, (size_t) k * N + base, t.aps.data() + (size_t) k * n, n);
     put(atom_tag, 3 * base, t.atom_tag.data(), 3 * n);
@@ -2045,7 +2173,6 @@ template <typename R> class Engine : public EngineBase {
       put(fm_slen, (size_t) g0 * nd, slen.data(), slen.size());
       put(fm_rf, (size_t) st0 * 32 * 4, P.rf.data(), P.rf.size());
       if (fm_coef_mode) put(fm_coef, (size_t) st0 * 32, P.cf.data(), P.cf.size());
-      CK(cudaStreamSynchronize(s0));
     }
     // run window: the next evaluation is this request's setup evaluation
     Slot &sl = slots[slot_id];
@@ -2065,8 +2192,8 @@ template <typename R> class Engine : public EngineBase {
     put(sys_seed, slot_id, &seed, 1);
     std::vector<int> rs(n, slot_id);
     put(res_sys, base, rs.data(), n);
-    CK(cudaStreamSynchronize(s0));
     set_thermostat_factors(3 * base, t.mass.data(), 3 * n);
+    put_wait();
     in.sys_res_begin[slot_id] = base;
     in.sys_res_end[slot_id] = base + n;
     in.ext_of[slot_id] = t.ext_of;
@@ -2111,56 +2238,34 @@ template <typename R> class Engine : public EngineBase {
   {
     if (!server) throw std::invalid_argument("not a serving handle");
     if (nsteps <= 0) return;
-    if (!graphs[0][0]) capture_steps(graphs[0][0], 1, false);
-    if (nsteps >= kChunk && !graphs[0][1]) capture_steps(graphs[0][1], kChunk, false);
+    capture_for(nsteps, 0);
     if (!ev_run0) {
       CK(cudaEventCreate(&ev_run0));
       CK(cudaEventCreate(&ev_run1));
     }
-    long long done = 0;
     CK(cudaEventRecord(ev_run0, s0));
-    while (nsteps - done >= kChunk) {
-      CK(cudaGraphLaunch(graphs[0][1], s0));
-      done += kChunk;
-    }
-    while (done < nsteps) {
-      CK(cudaGraphLaunch(graphs[0][0], s0));
-      done++;
-    }
+    launch_steps(nsteps, 0);
     CK(cudaEventRecord(ev_run1, s0));
+    CK(cudaMemcpyAsync(h_call.p, nl.p, sizeof(dev::NLState), cudaMemcpyDeviceToHost, s0));
     CK(cudaStreamSynchronize(s0));
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, ev_run0, ev_run1));
     last_run_ms = ms;
     step += nsteps;
-    check_list();
+    check_state(*h_call.at<dev::NLState>(0));
   }
 
   void release(int k) override
   {
     check_slot(k);
     Slot &sl = slots[k];
-    const int base = sl.base, n = sl.n_res, N = n_res_cap();
-    (void) N;
-    fill(res_sys, base, n, -1);
-    fill(res_flags, base, n, (int) (R_FIRST | R_LAST));
-    fill(res_chain, base, n, -1);
-    fill(excl_self, base, n, 0x1ffu);
-    fill(excl_next, base, n, 0u);
-    fill(bond_i, (size_t) 4 * base, (size_t) 4 * n, -1);
-    fill(x, (size_t) 9 * base, (size_t) 9 * n, 0.0);
-    fill(v, (size_t) 9 * base, (size_t) 9 * n, 0.0);
-    const int nd = in.ff.p.fm_nd;
-    if (nd > 0) {
-      fill(fm_slen, (size_t) (base / 32) * nd, (size_t) sl.groups * nd, 0);
-      fill(fm_soff, (size_t) (base / 32) * nd, (size_t) sl.groups * nd, 0);
-    }
-    int zero = 0;
-    dev::SlotRun w{0, 0, 0, 0.0, 0.0};
-    put(sys_begin, k, &zero, 1);
-    put(sys_end, k, &zero, 1);
-    put(slot_run, k, &w, 1);
-    CK(cudaStreamSynchronize(s0));
+    const int base = sl.base, n = sl.n_res, nd = in.ff.p.fm_nd;
+    // its residues back to residues of no request, its window and range to none
+    dev::k_release<<<(n + 127) / 128, 128, 0, s0>>>(
+        dev::ReleaseArgs{res_sys.p, res_flags.p, res_chain.p, bond_i.p, fm_slen.p, fm_soff.p, excl_self.p, excl_next.p, x.p,
+                         v.p, sys_begin.p, sys_end.p, slot_run.p, base, n, k, nd > 0 ? base / 32 * nd : 0,
+                         nd > 0 ? sl.groups * nd : 0});
+    CK(cudaGetLastError());
     give_range(free_groups, base / 32, sl.groups);
     give_range(free_stripes, sl.stripe0, sl.stripes);
     in.sys_res_begin[k] = in.sys_res_end[k] = 0;
@@ -2196,7 +2301,7 @@ template <typename R> class Engine : public EngineBase {
     auto add = [&](const auto &buf) { b += (long long) (buf.n * sizeof(*buf.p)); };
     add(res_type), add(res_flags), add(res_chain), add(chain_start), add(chain_end), add(atom_tag), add(atom_type);
     add(aps), add(tables), add(x), add(v), add(mass), add(g1), add(g2), add(ftot), add(work), add(e_res), add(energy);
-    add(pos), add(cpos), add(rrec), add(cb_build), add(facc), add(pairs), add(ncount), add(hbq), add(dacc), add(e_fix), add(nl), add(dstep);
+    add(perm), add(stage), add(pos), add(cpos), add(rrec), add(cb_build), add(facc), add(pairs), add(ncount), add(hbq), add(dacc), add(e_fix), add(nl), add(dstep);
     add(ev_pref), add(ev_cs), add(ev_cl), add(excl_self), add(excl_next), add(bond_i), add(bond_j), add(bond_k);
     add(bond_r0), add(fm_soff), add(fm_slen), add(fm_rf), add(fm_coef), add(tb_data), add(tb_present);
     add(go_start), add(go_partner), add(go_rnat), add(go_gamma), add(go_sig_sq), add(go_norm);

@@ -2169,6 +2169,37 @@ __global__ void k_continue(StepArgs<R> a, const Integrator *inp, const double *f
   }
 }
 
+// A finished request leaves a serving handle: its residues [base, base + n)
+// become residues of no request (flagged chain ends of no chain, fully
+// excluded, no bonds, at rest at the origin), its memory blocks empty, its
+// window and residue range none.
+struct ReleaseArgs {
+  int *res_sys, *res_flags, *res_chain, *bond_i, *fm_slen, *fm_soff;
+  unsigned *excl_self, *excl_next;
+  double *x, *v;
+  int *sys_begin, *sys_end;
+  SlotRun *slot_run;
+  int base, n, slot, fm0, fm_n;
+};
+__global__ void k_release(ReleaseArgs q)
+{
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, nthr = gridDim.x * blockDim.x;
+  if (t < q.n) {
+    q.res_sys[q.base + t] = -1;
+    q.res_flags[q.base + t] = (int) (R_FIRST | R_LAST);
+    q.res_chain[q.base + t] = -1;
+    q.excl_self[q.base + t] = 0x1ffu;
+    q.excl_next[q.base + t] = 0u;
+  }
+  for (int k = t; k < 4 * q.n; k += nthr) q.bond_i[(size_t) 4 * q.base + k] = -1;
+  for (int k = t; k < 9 * q.n; k += nthr) q.x[(size_t) 9 * q.base + k] = q.v[(size_t) 9 * q.base + k] = 0.0;
+  for (int k = t; k < q.fm_n; k += nthr) q.fm_slen[q.fm0 + k] = q.fm_soff[q.fm0 + k] = 0;
+  if (t == 0) {
+    q.sys_begin[q.slot] = q.sys_end[q.slot] = 0;
+    q.slot_run[q.slot] = SlotRun{0, 0, 0, 0.0, 0.0};
+  }
+}
+
 // Caller-order staging <-> internal order: out[a] = in[perm[a]] / out[perm[a]] = in[a]
 __global__ void k_gather3(const double *in, const int *perm, int n, double *out)
 {
@@ -2186,12 +2217,19 @@ __global__ void k_scatter3(const double *in, const int *perm, int n, double *out
   for (int c = 0; c < 3; c++) out[3 * p + c] = in[3 * a + c];
 }
 
-// Conservative total force of the last evaluation in FP64 (no Langevin)
-template <typename R> __global__ void k_total_force(StepArgs<R> a, double *ftot)
+// Conservative total force of the last evaluation in FP64 (no Langevin), in
+// internal order and, through perm, in the caller's
+template <typename R> __global__ void k_total_force(StepArgs<R> a, double *ftot, const int *perm, double *f_ext)
 {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= 3 * a.n_atoms) return;
-  ftot[k] = (double) (long long) a.s.facc[k] * F_UNSCALE;
+  if (k >= a.n_atoms) return;
+  const int q = perm[k];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const double f = (double) (long long) a.s.facc[3 * (size_t) k + c] * F_UNSCALE;
+    ftot[3 * (size_t) k + c] = f;
+    f_ext[3 * (size_t) q + c] = f;
+  }
 }
 
 // Thermo row of the current step: [fix total, vexcluded, bonds, kinetic],

@@ -255,8 +255,8 @@ class AwsemSystem:
                                                   None if va is None else _ptr(va)), "awsem_set_state")
 
     def get_state(self):
-        x = np.zeros((self.natoms, 3))
-        v = np.zeros((self.natoms, 3))
+        x = np.empty((self.natoms, 3))
+        v = np.empty((self.natoms, 3))
         _check(self.lib, self.lib.awsem_get_state(self.h, _ptr(x), _ptr(v)), "awsem_get_state")
         return x, v
 
@@ -274,7 +274,7 @@ class AwsemSystem:
         return e
 
     def forces(self) -> np.ndarray:
-        f = np.zeros((self.natoms, 3))
+        f = np.empty((self.natoms, 3))
         _check(self.lib, self.lib.awsem_forces(self.h, _ptr(f)), "awsem_forces")
         return f
 
@@ -441,7 +441,7 @@ class AwsemBatch(AwsemSystem):
 
     def get_state(self, r: int = 0):
         n = self.replica_natoms(r)
-        x, v = np.zeros((n, 3)), np.zeros((n, 3))
+        x, v = np.empty((n, 3)), np.empty((n, 3))
         _check(self.lib, self.lib.awsem_replica_get_state(self.h, r, _ptr(x), _ptr(v)), "awsem_replica_get_state")
         return x, v
 
@@ -468,14 +468,14 @@ class AwsemBatch(AwsemSystem):
 
     def get_state_all(self, x: np.ndarray | None = None, v: np.ndarray | None = None):
         """Every replica at once into x, v (allocated when not given)."""
-        x = np.zeros((self.natoms, 3)) if x is None else x
-        v = np.zeros((self.natoms, 3)) if v is None else v
+        x = np.empty((self.natoms, 3)) if x is None else x
+        v = np.empty((self.natoms, 3)) if v is None else v
         assert x.flags.c_contiguous and v.flags.c_contiguous and x.dtype == np.float64 and v.dtype == np.float64
         _check(self.lib, self.lib.awsem_batch_get_state(self.h, _ptr(x), _ptr(v)), "awsem_batch_get_state")
         return x, v
 
     def forces(self, r: int = 0) -> np.ndarray:
-        f = np.zeros((self.replica_natoms(r), 3))
+        f = np.empty((self.replica_natoms(r), 3))
         _check(self.lib, self.lib.awsem_replica_forces(self.h, r, _ptr(f)), "awsem_replica_forces")
         return f
 
@@ -581,7 +581,7 @@ class AwsemServer:
 
     def collect(self, slot: int):
         n = self.natoms.pop(slot)
-        x, v, e = np.zeros((n, 3)), np.zeros((n, 3)), np.zeros(21)
+        x, v, e = np.empty((n, 3)), np.empty((n, 3)), np.empty(21)
         _check(self.lib, self.lib.awsem_server_collect(self.h, slot, _ptr(x), _ptr(v), _ptr(e)),
                "awsem_server_collect")
         return x, v, e
