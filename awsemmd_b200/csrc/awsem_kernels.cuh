@@ -117,6 +117,15 @@ struct __align__(64) RadRec {
   int type, flags, chain, pad;
 };
 static_assert(sizeof(RadRec) == 64 && offsetof(RadRec, type) == 48, "RadRec layout");
+// a record, in two 32-byte loads
+__device__ __forceinline__ RadRec load_rec(const RadRec *p)
+{
+  const Word4 u = reinterpret_cast<const Word4 *>(p)[0], v = reinterpret_cast<const Word4 *>(p)[1];
+  RadRec r;
+  r.sw = u.x, r.bur = u.y, r.x1 = u.z, r.x2 = u.w, r.sigp = v.x, r.pad0 = 0.0;
+  r.type = __double2loint(v.z), r.flags = __double2hiint(v.z), r.chain = __double2loint(v.w), r.pad = 0;
+  return r;
+}
 
 template <typename R> struct StepArgs {
   DevSys<R> s;
@@ -325,14 +334,15 @@ template <typename R, int BLOCK> struct PrepareTile {
     const int r = r0 + (int) threadIdx.x, here = min(BLOCK, a.n_run - r0);
     if (on) {
       double4 *w = const_cast<double4 *>(a.s.pos) + (size_t) r * N_BEADS;
-      w[B_CA] = make_double4(ca[0], ca[1], ca[2], 0.0);
+      const double info = pack_info(a.s.res_chain[r], a.s.res_type[r], a.s.res_flags[r]);
+      w[B_CA] = make_double4(ca[0], ca[1], ca[2], info);
       w[B_CB] = make_double4(cb[0], cb[1], cb[2], 0.0);
       w[B_O] = make_double4(o[0], o[1], o[2], 0.0);
       w[B_N] = make_double4(n[0], n[1], n[2], 0.0);
       w[B_H] = make_double4(h[0], h[1], h[2], 0.0);
       w[B_CP] = make_double4(cp[0], cp[1], cp[2], 0.0);
       const_cast<double4 *>(a.s.cpos)[r] =
-          gly ? make_double4(ca[0], ca[1], ca[2], 0.0) : make_double4(cb[0], cb[1], cb[2], 0.0);
+          gly ? make_double4(ca[0], ca[1], ca[2], info) : make_double4(cb[0], cb[1], cb[2], info);
       if (over) a.lst_over[a.res_sys[r]] = 1;
     }
     for (int k = threadIdx.x; k < 9 * here; k += BLOCK) a.s.facc[(size_t) 9 * r0 + k] = 0ull;
@@ -469,7 +479,13 @@ template <typename R> __global__ void __launch_bounds__(kPrepBlock) k_prepare(St
 // contact bead of residue r (one load, no dependence on the residue's flags)
 template <typename R> __device__ __forceinline__ V3<double> contact(const DevSys<R> &s, int r)
 {
-  const double4 q = s.cpos[r];
+  const Word4 q = load4(s.cpos + r);
+  return {q.x, q.y, q.z};
+}
+template <typename R> __device__ __forceinline__ V3<double> contact(const DevSys<R> &s, int r, ResInfo &info)
+{
+  const Word4 q = load4(s.cpos + r);
+  info = unpack_info(q.w);
   return {q.x, q.y, q.z};
 }
 
@@ -703,15 +719,20 @@ template <typename R> __global__ void k_nl_build(StepArgs<R> a, GridArgs g, int 
   nl_build_pass(a, g, n_launch, grid_span());
 }
 
-// Pairs of the list, grid-stride (the count is known only on the device)
-#define FOR_EACH_PAIR(a, p, sp) \
-  for (int p = (sp).t, np_ = min((a).nl->npairs, (a).pcap); p < np_; p += (sp).nthr)
 // Pairs of the near list (written by the density pass of this evaluation):
 // index p is entry p % seg_len of segment p / seg_len, present when below
-// that segment's count
-#define FOR_EACH_NEAR_PAIR(a, p, sp)                                                                     \
-  for (int p = (sp).t, S_ = (a).nl->seg_len, end_ = (a).nl->nseg * S_; p < end_; p += (sp).nthr)      \
-    if (p - (p / S_) * S_ < (a).seg_n[p / S_])
+// that segment's count.  The pair is loaded beside the count.  (Loading the
+// next pair ahead of the current one's work cost the registers that k_radial
+// does not have: 93 -> 99 us on 283,000 residues.)
+template <typename R, class F> __device__ __forceinline__ void for_each_near_pair(const StepArgs<R> &a, Span sp, F &&visit)
+{
+  const int len = a.nl->seg_len, end = a.nl->nseg * len;
+  for (int p = sp.t; p < end; p += sp.nthr) {
+    const int sg = p / len, cnt = a.seg_n[sg];
+    const int2 ij = p < a.pcap ? a.cpairs[p] : make_int2(0, 0);  // the last segment may reach past the list
+    if (p - sg * len < cnt) visit(ij.x, ij.y);
+  }
+}
 
 // Density well value (FP64 in both forms).  The plain FP64 form evaluates
 // the reference's 0.25 (1 + tanh(kappa (r - rmin))) (1 + tanh(kappa (rmax -
@@ -764,16 +785,18 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void density_
     int2 ij = {0, 0};
     double rsq = 0.0;
     bool near = false;
+    ResInfo wi{}, wj{};
     if (q < hi) {
       ij = a.pairs[q];
-      rsq = norm2(diff<double>(contact(s, ij.x), contact(s, ij.y)));
+      const V3<double> ci = contact(s, ij.x, wi), cj = contact(s, ij.y, wj);
+      rsq = norm2(diff<double>(ci, cj));
       near = rsq < need_sq;
     }
     const unsigned m = __ballot_sync(0xffffffffu, near);
     if (near) a.cpairs[lo + cnt + __popc(m & ((1u << lane) - 1u))] = ij;
     cnt += __popc(m);
     const int i = ij.x, j = ij.y;
-    if (q >= hi || (s.res_chain[j] == s.res_chain[i] && j - i <= 1)) continue;
+    if (q >= hi || (wj.chain == wi.chain && j - i <= 1)) continue;
     const double r = sqrt(rsq);
     if (water && rsq > p.w_rmin_sq[0] && rsq < p.w_rmax_sq[0]) {
       const double th = density_well<R>(r, p.w_rmin_th[0], p.w_rmax_th[0], p.water_kappa, p.well_rmin[0], p.well_rmax[0]);
@@ -1189,13 +1212,10 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void water_xi
   if (!(p.terms & T_WATER) || !(a.groups & G_FIX)) return;
   unsigned long long *acc = (unsigned long long *) a.dacc + (size_t) 2 * s.n_res;
   const double *WG = s.tables + TB_WATER;
-  FOR_EACH_NEAR_PAIR(a, q, sp)
-  {
-    const int2 ij = a.cpairs[q];
-    const int i = ij.x, j = ij.y;
+  for_each_near_pair(a, sp, [&](int i, int j) {
     // the residues' packed records (written by the residue pass) and contact beads
-    const RadRec ri = a.rrec[i], rj = a.rrec[j];
-    if (rj.chain == ri.chain && j - i < p.contact_cutoff) continue;
+    const RadRec ri = load_rec(a.rrec + i), rj = load_rec(a.rrec + j);
+    if (rj.chain == ri.chain && j - i < p.contact_cutoff) return;
     const R rsq = norm2(diff<R>(contact(s, i), contact(s, j)));
     const int ti = ri.type, tj = rj.type;
     // pairs with a phosphorylated residue use the phosphorylation gammas (fix_backbone.cpp:2872-2885)
@@ -1214,7 +1234,7 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void water_xi
         atomicAdd(acc + j, (unsigned long long) fix_dens(tg * ri.sw));
       }
     }
-  }
+  });
 }
 
 template <typename R> __global__ void k_water_xi(StepArgs<R> a, FFParams p) { water_xi_pass(a, p, grid_span()); }
@@ -1249,13 +1269,10 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void radial_p
   const uint32_t T = p.terms;
   const int dh = p.helix_i_diff;
   unsigned long long *e_water = (unsigned long long *) a.e_fix + (size_t) 3 * n;
-  FOR_EACH_NEAR_PAIR(a, q, sp)
-  {
-    const int2 ij = a.cpairs[q];
-    const int i = ij.x, j = ij.y;
+  for_each_near_pair(a, sp, [&](int i, int j) {
     // every per-residue input of the pair, loaded up front and without
     // conditions, so that the gathers are in flight together
-    const RadRec ri = a.rrec[i], rj = a.rrec[j];
+    const RadRec ri = load_rec(a.rrec + i), rj = load_rec(a.rrec + j);
     const V3<double> c_i = contact(s, i), c_j = contact(s, j);
     const double ui = (double) a.dacc[(size_t) 2 * n + i], uj = (double) a.dacc[(size_t) 2 * n + j];
     const int fli = ri.flags, flj = rj.flags, ti = ri.type, tj = rj.type;
@@ -1326,7 +1343,7 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void radial_p
         scatter_fix(s, j, gj ? B_CA : B_CB, g);
       }
     }
-  }
+  });
 }
 
 // blocks per SM the radial and detection passes are compiled for (the
@@ -1416,10 +1433,11 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void pair_pas
     if (q >= 0) {
       const int2 ij = list[q];
       i = ij.x, j = ij.y;
-      const bool shortr = s.res_chain[j] == s.res_chain[i] && j - i < 5;
+      ResInfo wi, wj;
+      dca = sqrtf((float) norm2(diff<R>(bead_ca(s, i, wi), bead_ca(s, j, wj))));
+      const bool shortr = wj.chain == wi.chain && j - i < 5;
       sh = shortr ? 0 : 9;
       const unsigned excl = j == i + 1 ? a.excl_next[i] : 0u;
-      dca = sqrtf((float) norm2(diff<R>(bead(s, i, B_CA), bead(s, j, B_CA))));
       mask = ~excl & 0x1ffu;
     }
 #pragma unroll
@@ -1470,16 +1488,15 @@ template <typename R, bool SEL = false> __device__ __forceinline__ void pair_pas
   // (a warp's 32 indices lie in one near-list segment: segments are multiples of 32 long)
   for (int base = sp.t - lane; base < np; base += sp.nthr) {
     const int q = base + lane, sg = base / seg, have = near ? a.seg_n[sg] - (base - sg * seg) : np - base;
+    const int2 ij = q < npairs ? list[q] : make_int2(0, 0);  // beside the segment's count
     if (have <= 0) continue;  // warp-uniform: past this segment's near pairs
     bool q_d0 = false, q_d1 = false, q_p = false, q_e = false;  // queue: DSSP O(i), DSSP O(j), P_AP; stage: EV
     if (lane < have) {
-    const int2 ij = list[q];
     const int i = ij.x, j = ij.y;
-    // (the topology arrays, not the residue pass's records: this pass runs
-    // beside the residue pass)
-    const int fli = s.res_flags[i], flj = s.res_flags[j];
-    const bool other = s.res_chain[j] != s.res_chain[i];
-    const V3<double> ca_i = bead(s, i, B_CA), ca_j = bead(s, j, B_CA);
+    ResInfo wi, wj;
+    const V3<double> ca_i = bead_ca(s, i, wi), ca_j = bead_ca(s, j, wj);
+    const int fli = wi.flags, flj = wj.flags;
+    const bool other = wj.chain != wi.chain;
     const int dij = j - i;
     const R rca2 = norm2(diff<R>(ca_i, ca_j));
     // excluded volume between beads of i and j: staged (below), so that the
