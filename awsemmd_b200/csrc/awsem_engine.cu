@@ -1243,6 +1243,7 @@ template <typename R> class Engine : public EngineBase {
     pair_blocks = sh[1];
     hb_blocks = sh[2];
     fm_grid = sh[3];
+    shapes_given = true;
     release_graphs();
   }
 
@@ -1324,6 +1325,7 @@ template <typename R> class Engine : public EngineBase {
   {
     if (server) throw std::invalid_argument("autotune: not available on a serving handle");
     if (reps <= 0) throw std::invalid_argument("reps must be positive");
+    shapes_given = true;
     const int na = natoms();
     DBuf<double> sx, sv;
     sx.alloc((size_t) 3 * na);
@@ -1545,14 +1547,8 @@ template <typename R> class Engine : public EngineBase {
     fm_slen.upload(slen, s0);
     fm_rf.upload(rf, s0);
     fm_coef.upload(cf, s0);
-    // enough warps to fill the GPU on small systems: split each group's
-    // separations over several warps when there are few groups
-    int sms = 148;
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    fm_dsplit = std::max(1, std::min(std::max(nd, 1), (16 * sms + fm_groups - 1) / std::max(fm_groups, 1)));
-    // FP64 rows are long enough to be units of their own at every size, and
-    // evenly sized units end together
-    if (sizeof(R) == 8) fm_dsplit = std::max(nd, 1);
+    CK(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device));
+    fm_default_shape(fm_groups);
     CK(cudaStreamSynchronize(s0));  // host vectors go out of scope
   }
 
@@ -1570,6 +1566,22 @@ template <typename R> class Engine : public EngineBase {
   // one warp per fragment-memory work unit, or a smaller persistent grid
   // (fm_grid blocks) whose warps loop over the units
   int fm_grid = 0;
+  bool shapes_given = false;  // by the caller or the autotuner: kept
+
+  // Default shapes for `groups` residue groups.  Separations split over enough
+  // warps to fill the multiprocessors, over two at least (units that end
+  // closer together: 1,024 chains 881 -> 860 us a step); FP64 rows are units
+  // of their own at every size.  FP32 units are taken by three blocks a
+  // multiprocessor: HBM is saturated (0.31 ms against 0.34 with a warp a unit
+  // on 1,858 MB) and the pair passes beside it find room (1,024 chains 925 ->
+  // 867 us a step, 40,000 residues 173 -> 171; two blocks 934 and 165).
+  void fm_default_shape(int groups)
+  {
+    if (shapes_given) return;
+    const int nd = std::max(in.ff.p.fm_nd, 1), g = std::max(groups, 1);
+    fm_dsplit = sizeof(R) == 8 ? nd : std::max(std::min(2, nd), std::min(nd, (16 * sms_ + g - 1) / g));
+    fm_grid = sizeof(R) == 8 ? 0 : 3 * sms_;
+  }
   int fm_blocks() const
   {
     const int all = fm_psplit(fm_groups) > 1 ? fm_units() : (fm_units() * 32 + 127) / 128;
@@ -2214,6 +2226,8 @@ template <typename R> class Engine : public EngineBase {
     int want = std::min(n(), std::max(4096, (hwm + 4095) / 4096 * 4096));
     if (want != launch_res) {
       launch_res = want;
+      // a handle made for millions of residues serves a few thousand with units of one separation
+      fm_default_shape((want + 31) / 32);
       release_graphs();
     }
   }
