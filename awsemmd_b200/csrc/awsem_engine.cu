@@ -809,15 +809,12 @@ template <typename R> class Engine : public EngineBase {
 
   void zero_unwritten_energies(int groups)
   {
-    // slots the selected groups do not write must read as zero
-    int nn = n();
-    if (!(groups & dev::G_FIX) || !(in.ff.p.terms & T_FM) || in.ff.p.fm_nd == 0)
-      CK(cudaMemsetAsync(e_res.p + (size_t) E_FRAGMEM * nn, 0, sizeof(double) * nn, s0));
+    // slots the selected groups do not write must read as zero (a term that the force field leaves off never writes)
+    const int nn = n();
     if (!(groups & dev::G_BOND)) CK(cudaMemsetAsync(e_res.p + (size_t) E_BOND * nn, 0, sizeof(double) * nn, s0));
-    if (!(groups & dev::G_FIX) || !(in.ff.p.terms & T_AMHGO))
-      CK(cudaMemsetAsync(e_res.p + (size_t) E_AMHGO * nn, 0, sizeof(double) * nn, s0));
     if (!(groups & dev::G_FIX))
-      for (int t : {E_SHAKE, E_MEMB, E_VFRAGMEM}) CK(cudaMemsetAsync(e_res.p + (size_t) t * nn, 0, sizeof(double) * nn, s0));
+      for (int t : {E_AMHGO, E_SHAKE, E_MEMB, E_VFRAGMEM})
+        CK(cudaMemsetAsync(e_res.p + (size_t) t * nn, 0, sizeof(double) * nn, s0));
   }
 
   // energy sums of replicas [rep0, rep0 + count) (all of them by default)
@@ -842,22 +839,28 @@ template <typename R> class Engine : public EngineBase {
   cudaGraphExec_t eval_graph = nullptr;
   int eval_groups = -1, eval_calls = 0;
 
+  // h_io: positions, step counter; then forces, energies, list state
+  DBuf<double> results;  // the same on the device
+  size_t io_in() const { return sizeof(double) * (3 * (size_t) natoms() + 1); }
+  size_t io_out() const { return sizeof(double) * (3 * (size_t) natoms() + E_SLOTS) + sizeof(dev::NLState); }
+  dev::NLState io_state() const
+  {
+    dev::NLState st;
+    std::memcpy(&st, h_io.p + io_in() + io_out() - sizeof st, sizeof st);
+    return st;
+  }
+
   void queue_evaluation(int groups)
   {
     const int na = natoms(), tb = 256, nb = (na + tb - 1) / tb;
-    const size_t bytes = sizeof(double) * 3 * na;
-    CK(cudaMemcpyAsync(stage.p, h_io.p, bytes, cudaMemcpyHostToDevice, s0));
-    CK(cudaMemcpyAsync(dstep.p, h_call.at<long long>(kHostStep), sizeof(long long), cudaMemcpyHostToDevice, s0));
-    dev::k_gather3<<<nb, tb, 0, s0>>>(stage.p, perm.p, na, x.p);
+    CK(cudaMemcpyAsync(stage.p, h_io.p, io_in(), cudaMemcpyHostToDevice, s0));
+    dev::k_inputs<<<nb, tb, 0, s0>>>(stage.p, perm.p, na, x.p, dstep.p);
     zero_unwritten_energies(groups);
     auto a = args(groups);
     launch_eval(a, false);
     if (lists_emulated()) dev::k_list_hold<R><<<(n_run() + 127) / 128, 128, 0, s0>>>(a);
-    dev::k_total_force<R><<<nb, tb, 0, s0>>>(a, ftot.p, perm.p, stage.p);
-    reduce_energies();
-    CK(cudaMemcpyAsync(h_io.p + bytes, stage.p, bytes, cudaMemcpyDeviceToHost, s0));
-    CK(cudaMemcpyAsync(h_call.p + kHostEnergy, energy.p, sizeof(double) * E_SLOTS, cudaMemcpyDeviceToHost, s0));
-    CK(cudaMemcpyAsync(h_call.p, nl.p, sizeof(dev::NLState), cudaMemcpyDeviceToHost, s0));
+    dev::k_results<R><<<E_SLOTS + nb, tb, 0, s0>>>(a, ftot.p, perm.p, results.p);
+    CK(cudaMemcpyAsync(h_io.p + io_in(), results.p, io_out(), cudaMemcpyDeviceToHost, s0));
   }
 
   void compute(long long st, const double *x_ext, double *f_ext, double *energies_out, int groups) override
@@ -866,10 +869,9 @@ template <typename R> class Engine : public EngineBase {
     if (server) throw std::invalid_argument("awsem_compute: not available on a serving handle");
     cont_step = -1;
     const int na = natoms();
-    const size_t bytes = sizeof(double) * 3 * na;
-    h_io.need(2 * bytes);
-    std::memcpy(h_io.p, x_ext, bytes);
-    *h_call.at<long long>(kHostStep) = st;
+    h_io.need(io_in() + io_out());
+    std::memcpy(h_io.p, x_ext, sizeof(double) * 3 * na);
+    *h_io.at<long long>(sizeof(double) * 3 * na) = st;
     step = st;
     if (lists_emulated()) {
       // the host's MD loop decides whether this evaluation's lists are new
@@ -900,14 +902,14 @@ template <typename R> class Engine : public EngineBase {
       // an evaluation whose pair list overflowed runs again on a grown list
       // (it changes no state, unless LAMMPS's lists are emulated, whose
       // per-step bookkeeping it advances: then the overflow is reported)
-      const int ovf = h_call.at<dev::NLState>(0)->overflow;
+      const int ovf = io_state().overflow;
       if (!ovf || attempt == 1 || lists_emulated()) break;
       grow_pairs(ovf);
     }
-    check_state(*h_call.at<dev::NLState>(0));
-    const double *f = reinterpret_cast<const double *>(h_io.p + bytes);
+    check_state(io_state());
+    const double *f = h_io.at<double>(io_in());
     for (int k = 0; k < 3 * na; k++) f_ext[k] += f[k];
-    if (energies_out) finish_energies(h_call.at<double>(kHostEnergy), energies_out, false);
+    if (energies_out) finish_energies(f + 3 * na, energies_out, false);
   }
 
   void release_eval_graph()
@@ -1010,6 +1012,7 @@ template <typename R> class Engine : public EngineBase {
     }
     perm.upload(pm, s0);
     stage.alloc((size_t) 6 * natoms());
+    if (n_sys() == 1) results.alloc(io_out() / sizeof(double));
     CK(cudaStreamSynchronize(s0));  // pm goes out of scope
   }
 
@@ -2315,7 +2318,7 @@ template <typename R> class Engine : public EngineBase {
     auto add = [&](const auto &buf) { b += (long long) (buf.n * sizeof(*buf.p)); };
     add(res_type), add(res_flags), add(res_chain), add(chain_start), add(chain_end), add(atom_tag), add(atom_type);
     add(aps), add(tables), add(x), add(v), add(mass), add(g1), add(g2), add(ftot), add(work), add(e_res), add(energy);
-    add(perm), add(stage), add(pos), add(cpos), add(rrec), add(cb_build), add(facc), add(pairs), add(ncount), add(hbq), add(dacc), add(e_fix), add(nl), add(dstep);
+    add(perm), add(stage), add(results), add(pos), add(cpos), add(rrec), add(cb_build), add(facc), add(pairs), add(ncount), add(hbq), add(dacc), add(e_fix), add(nl), add(dstep);
     add(ev_pref), add(ev_cs), add(ev_cl), add(excl_self), add(excl_next), add(bond_i), add(bond_j), add(bond_k);
     add(bond_r0), add(fm_soff), add(fm_slen), add(fm_rf), add(fm_coef), add(tb_data), add(tb_present);
     add(go_start), add(go_partner), add(go_rnat), add(go_gamma), add(go_sig_sq), add(go_norm);

@@ -2234,21 +2234,6 @@ __global__ void k_scatter3(const double *in, const int *perm, int n, double *out
   for (int c = 0; c < 3; c++) out[3 * p + c] = in[3 * a + c];
 }
 
-// Conservative total force of the last evaluation in FP64 (no Langevin), in
-// internal order and, through perm, in the caller's
-template <typename R> __global__ void k_total_force(StepArgs<R> a, double *ftot, const int *perm, double *f_ext)
-{
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.n_atoms) return;
-  const int q = perm[k];
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const double f = (double) (long long) a.s.facc[3 * (size_t) k + c] * F_UNSCALE;
-    ftot[3 * (size_t) k + c] = f;
-    f_ext[3 * (size_t) q + c] = f;
-  }
-}
-
 // Thermo row of the current step: [fix total, vexcluded, bonds, kinetic],
 // residue sums in a fixed tree order (one block of 256 threads).
 __global__ void k_thermo(const double *e_res, const long long *e_fix, int efix_slots, int n_res, const long long *step,
@@ -2337,10 +2322,10 @@ __global__ void k_q_sum(const double *partial, int n, double qnorm, double *out)
 
 // Per-term sums of each replica's residues in a fixed tree order
 // (block (t, r) sums energy slot t of replica rep0 + r)
-__global__ void k_energy_reduce(const double *e_res, const long long *e_fix, int efix_slots, int n_res,
-                                const int *sys_begin, const int *sys_end, double *out, int rep0)
+// energy slot t summed over residues [r0, r1) in a fixed tree order (a block of 256 threads; thread 0 has the sum)
+__device__ __forceinline__ double energy_slot(const double *e_res, const long long *e_fix, int efix_slots, int n_res, int t,
+                                              int r0, int r1)
 {
-  const int t = blockIdx.x, rep = rep0 + blockIdx.y;
   __shared__ double sh[256];
   double acc = 0.0;
   // pair-summed energies are kept in fixed point (e_fix slots)
@@ -2348,7 +2333,7 @@ __global__ void k_energy_reduce(const double *e_res, const long long *e_fix, int
               : t == E_SSB ? 5 : t == E_DH ? 6 : t == E_CONT_REST ? 7 : -1;
   if (k >= efix_slots) k = -1;
   const long long *fx = k >= 0 ? e_fix + (size_t) k * n_res : nullptr;
-  for (int r = sys_begin[rep] + threadIdx.x; r < sys_end[rep]; r += blockDim.x)
+  for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x)
     acc += e_res[(size_t) t * n_res + r] + (fx ? (double) fx[r] * F_UNSCALE : 0.0);
   sh[threadIdx.x] = acc;
   __syncthreads();
@@ -2356,7 +2341,53 @@ __global__ void k_energy_reduce(const double *e_res, const long long *e_fix, int
     if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[(size_t) rep * E_SLOTS + t] = sh[0];
+  return sh[0];
+}
+
+__global__ void k_energy_reduce(const double *e_res, const long long *e_fix, int efix_slots, int n_res,
+                                const int *sys_begin, const int *sys_end, double *out, int rep0)
+{
+  const int t = blockIdx.x, rep = rep0 + blockIdx.y;
+  const double e = energy_slot(e_res, e_fix, efix_slots, n_res, t, sys_begin[rep], sys_end[rep]);
+  if (threadIdx.x == 0) out[(size_t) rep * E_SLOTS + t] = e;
+}
+
+// The results of a force call on a single system, side by side for one copy
+// to the host: forces in the caller's order (and in internal order to ftot;
+// conservative, no Langevin), the energy slots, and the list state with its
+// error flags.  E_SLOTS blocks for the energies, then blocks of 256 atoms.
+template <typename R>
+__global__ void __launch_bounds__(256) k_results(StepArgs<R> a, double *ftot, const int *perm, double *out)
+{
+  if (blockIdx.x < E_SLOTS) {
+    const double e = energy_slot(a.e_res, a.e_fix, a.efix_slots, a.s.n_res, blockIdx.x, 0, a.s.n_res);
+    if (threadIdx.x == 0) out[3 * (size_t) a.n_atoms + blockIdx.x] = e;
+    return;
+  }
+  const int k = (blockIdx.x - E_SLOTS) * 256 + threadIdx.x;
+  if (blockIdx.x == E_SLOTS) {
+    int *to = reinterpret_cast<int *>(out + 3 * (size_t) a.n_atoms + E_SLOTS);
+    for (int w = threadIdx.x; w < (int) (sizeof(NLState) / 4); w += 256) to[w] = reinterpret_cast<const int *>(a.nl)[w];
+  }
+  if (k >= a.n_atoms) return;
+  const int q = perm[k];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const double f = (double) (long long) a.s.facc[3 * (size_t) k + c] * F_UNSCALE;
+    ftot[3 * (size_t) k + c] = f;
+    out[3 * (size_t) q + c] = f;
+  }
+}
+
+// ... and its inputs: positions in the caller's order, then the step counter
+__global__ void k_inputs(const double *in, const int *perm, int n, double *x, long long *step)
+{
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k == 0) *step = __double_as_longlong(in[3 * (size_t) n]);
+  if (k >= n) return;
+  const int q = perm[k];
+#pragma unroll
+  for (int c = 0; c < 3; c++) x[3 * (size_t) k + c] = in[3 * (size_t) q + c];
 }
 
 }  // namespace dev
