@@ -782,7 +782,7 @@ template <typename R> class Engine : public EngineBase {
   }
 
   // The residue and backbone kernels: by tasks while a wave of blocks (four per multiprocessor) covers the residues.
-  // At 17,000 residues (540 blocks) the two take 35 us by tasks and 41 by residues, at 40,000 61 and 44.
+  // At 17,000 residues (540 blocks) the two take 34 us by tasks and 41 by residues, at 40,000 61 and 46.
   bool by_tasks() const { return task_blocks() <= 4 * sms_; }
   void launch_residue(const dev::StepArgs<R> &a, cudaStream_t s)
   {

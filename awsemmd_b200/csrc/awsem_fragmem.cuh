@@ -247,7 +247,7 @@ template <typename R> struct FMSums {
   R es = 0, fs[4] = {0, 0, 0, 0}, es1 = 0, fs1[4] = {0, 0, 0, 0};  // even and odd records
   R et = 0, ft[4] = {0, 0, 0, 0};                                  // FP64: the row's pieces so far
   long long fca[3] = {0, 0, 0}, fcb[3] = {0, 0, 0};
-  double e = 0.0;
+  long long e = 0;  // fixed point by row: the same whatever rows share a unit
 
   // a piece ends
   __device__ __forceinline__ void end_piece()
@@ -270,7 +270,7 @@ template <typename R> struct FMSums {
   __device__ __forceinline__ void end_row(R scale, R s2, const R r[4], const V3<R> dv[4], const Pos &pos, int ii,
                                           bool live, int j, unsigned long long *facc)
   {
-    e += (double) (scale * et);
+    e += fix_force((double) (scale * et));
     long long fja[3] = {0, 0, 0}, fjb[3] = {0, 0, 0};
     if constexpr (sizeof(R) == 8) {
       V3<R> dp[4];
@@ -322,7 +322,7 @@ template <typename R> struct FMSums {
       red_add3(facc + (size_t) 9 * i, fca);
       red_add3(facc + (size_t) 9 * i + 3, fcb);
     }
-    long long en = live ? fix_force(e) : 0;
+    long long en = live ? e : 0;
     if (e_stride) {
       if (en) atomicAdd(e_acc + (size_t) i * e_stride, (unsigned long long) en);
     } else {
