@@ -868,7 +868,8 @@ def main():
         torch.cuda.empty_cache()  # the serving handle takes the memory budget
         served = serving_bench(args, dist, tmp)
     from awsemmd_b200.engine import NKERNELS
-    launches = NKERNELS * (md + 1) * args.steps  # every kernel of every MD step (setup evaluation included)
+    # every kernel of every MD step (setup evaluation included); the list decision is part of the prepare kernel
+    launches = (NKERNELS - 1) * (md + 1) * args.steps
     if dist.rank == 0:
         line = {"metric": "residue-steps/s", "value": value, "unit": "residue-steps/s", "n_gpus": dist.world,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": total_ms / args.steps,
