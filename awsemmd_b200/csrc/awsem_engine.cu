@@ -30,12 +30,15 @@ struct StateError : std::runtime_error {
   using std::runtime_error::runtime_error;
 };
 
+// A failed call is reported once: its error does not stay behind for the next call's cudaGetLastError.
 #define CK(call)                                                                                 \
   do {                                                                                           \
     cudaError_t e_ = (call);                                                                     \
-    if (e_ != cudaSuccess)                                                                       \
+    if (e_ != cudaSuccess) {                                                                     \
+      cudaGetLastError();                                                                        \
       throw CudaError(std::string(#call) + ": " + cudaGetErrorString(e_) + " (" __FILE__ ":" + \
                       std::to_string(__LINE__) + ")");                                           \
+    }                                                                                            \
   } while (0)
 
 template <typename T> struct DBuf {
@@ -884,13 +887,11 @@ template <typename R> class Engine : public EngineBase {
     }
     eval_calls++;
     if (eval_calls >= 3 && !eval_graph && !sel_cap) {
-      cudaGraph_t graph;
-      CK(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
-      queue_evaluation(groups);
-      CK(cudaStreamEndCapture(s0, &graph));
-      set_node_priorities(graph);
-      CK(cudaGraphInstantiate(&eval_graph, graph, 0));
-      CK(cudaGraphDestroy(graph));
+      try {
+        record(eval_graph, [&] { queue_evaluation(groups); });
+      } catch (const CudaError &) {
+        eval_calls = 0;  // e.g. no memory for the graph: this call and the next two are queued directly
+      }
     }
     for (int attempt = 0; attempt < 2; attempt++) {
       if (eval_graph && !sel_cap)
@@ -1125,22 +1126,41 @@ template <typename R> class Engine : public EngineBase {
     int nn = n(), tb = 128, nb = (n_run() + tb - 1) / tb;
     const bool persistent = step_form == 1;
     if (persistent) prepare_persistent(a);
-    cudaGraph_t graph;
-    CK(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
-    for (int c = 0; c < count; c++) {
-      if (persistent) {
-        launch_step_persistent(a);
-      } else {
-        launch_eval(a, true);
-        dev::k_finish<R><<<finish_blocks(), dev::kFinishThreads, 0, s0>>>(a, d_integ.p, g1.p, g2.p, ftot.p, x.p);
+    record(exec, [&] {
+      for (int c = 0; c < count; c++) {
+        if (persistent) {
+          launch_step_persistent(a);
+        } else {
+          launch_eval(a, true);
+          dev::k_finish<R><<<finish_blocks(), dev::kFinishThreads, 0, s0>>>(a, d_integ.p, g1.p, g2.p, ftot.p, x.p);
+        }
+        if (thermo)
+          dev::k_thermo<<<n_sys(), 256, 0, s0>>>(e_res.p, e_fix.p, efix_slots, nn, dstep.p, d_integ.p, sys_begin.p,
+                                                 sys_end.p, thermo_nrows, thermo_rows.p);
       }
-      if (thermo)
-        dev::k_thermo<<<n_sys(), 256, 0, s0>>>(e_res.p, e_fix.p, efix_slots, nn, dstep.p, d_integ.p, sys_begin.p, sys_end.p,
-                                               thermo_nrows, thermo_rows.p);
+    });
+  }
+
+  // What queue() puts on s0 and the streams that fork from it, as a graph.  A
+  // call that fails on the way ends the capture and drops the partial graph
+  // before it is reported, so that the streams take work again.
+  template <class Queue> void record(cudaGraphExec_t &exec, Queue &&queue)
+  {
+    cudaGraph_t graph = nullptr;
+    CK(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
+    try {
+      queue();
+      CK(cudaGetLastError());
+      CK(cudaStreamEndCapture(s0, &graph));
+      set_node_priorities(graph);
+      CK(cudaGraphInstantiate(&exec, graph, 0));
+    } catch (...) {
+      exec = nullptr;
+      if (!graph) cudaStreamEndCapture(s0, &graph);  // (again, and in vain, where ending it was what failed)
+      if (graph) cudaGraphDestroy(graph);
+      cudaGetLastError();
+      throw;
     }
-    CK(cudaStreamEndCapture(s0, &graph));
-    set_node_priorities(graph);
-    CK(cudaGraphInstantiate(&exec, graph, 0));
     CK(cudaGraphDestroy(graph));
   }
 

@@ -1,0 +1,72 @@
+"""The engine's host code on a CUDA runtime without a device
+(fake_cudart.cpp, preloaded into a child process): what its calls queue, record
+and wait for, and what they leave behind when a runtime call fails."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+PRELUDE = """
+import ctypes, sys, tempfile
+sys.path.insert(0, {root!r})
+from awsemmd_b200 import engine, synth
+fake = ctypes.CDLL({lib!r})
+for name in ("pending", "capturing", "graphs", "execs", "instantiated", "waits"):
+    getattr(fake, "fake_" + name).restype = ctypes.c_longlong
+ff = synth.forcefield_dir(tempfile.mkdtemp(dir={tmp!r}))
+def chain(n, seed=1):
+    return synth.chain_arrays(n, seed, n_mem_per_window=2)
+def system(n=20, precision="fp64"):
+    return engine.AwsemBatch.from_arrays(ff, [chain(n)], precision=precision)
+def refused(call):
+    try:
+        call()
+    except engine.AwsemError:
+        return True
+    return False
+"""
+
+
+@pytest.fixture(scope="module")
+def host(gpu_lib, tmp_path_factory):
+    d = tmp_path_factory.mktemp("host")
+    lib = str(d / "fake_cudart.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-o", lib, os.path.join(HERE, "fake_cudart.cpp")], check=True)
+
+    def run(script):
+        code = PRELUDE.format(root=os.path.dirname(HERE), lib=lib, tmp=str(d)) + script
+        r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LD_PRELOAD=lib), capture_output=True, text=True,
+                           timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+
+    return run
+
+
+@pytest.mark.parametrize("what,call", [("compute", "cudaMemcpyAsync"), ("compute", "cudaEventRecord"),
+                                       ("compute", "cudaLaunchKernel"), ("compute", "cudaGraphInstantiate"),
+                                       ("run", "cudaEventRecord"), ("run", "cudaLaunchKernel"),
+                                       ("run", "cudaGraphInstantiate")])
+def test_failed_recording(what, call, host):
+    """A runtime call that fails while a call's graph is recorded: the capture
+    is over, no graph is left behind, a force call is evaluated without one,
+    and the next call works."""
+    host(f"""
+what, call = {what!r}, {call!r}.encode()
+s = system()
+x = s.get_state(0)[0]
+one = (lambda: s.compute(x)) if what == "compute" else (lambda: s.run(30))
+for after in range({{b"cudaMemcpyAsync": 2, b"cudaGraphInstantiate": 1}}.get(call, 3)):
+    s.set_launch_shapes((1, 148, 148, 0))  # drops what is recorded
+    fake.fake_fail(call, after)
+    for k in range(100):
+        no = refused(one)
+        assert fake.fake_capturing() == 0 and fake.fake_graphs() == 0, (after, k)
+        if fake.fake_failed(call):
+            break
+    assert fake.fake_failed(call), after
+    assert no == (what == "run"), after
+    assert not refused(one), after
+""")
