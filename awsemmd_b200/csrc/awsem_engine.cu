@@ -125,6 +125,7 @@ class EngineBase {
     reps.clear();  // host copies are no longer needed: state lives on the device
   }
   virtual void setup() = 0;
+  virtual void settle() noexcept = 0;  // waits for what is queued (after a failed call)
   virtual void compute(long long step, const double *x_ext, double *f_ext, double *energies, int groups) = 0;
   virtual void set_state(int rep, const double *x_ext, const double *v_ext) = 0;
   virtual void get_state(int rep, double *x_ext, double *v_ext) = 0;
@@ -269,6 +270,13 @@ template <typename R> class Engine : public EngineBase {
     if (s1) cudaStreamDestroy(s1);
     if (s2) cudaStreamDestroy(s2);
     if (s3) cudaStreamDestroy(s3);
+  }
+
+  void settle() noexcept override
+  {
+    cudaStreamSynchronize(s0);
+    cudaGetLastError();
+    adm_used = 0;
   }
 
   int n() const { return in.top.n_res; }
@@ -2377,11 +2385,19 @@ struct DeviceRestore {
   }
 };
 
-template <typename Fn> static int guarded(Fn fn)
+// Runs an entry point's work and turns its exceptions into codes.  A call that
+// queues copies on the buffers its handle keeps gives the handle: what a call
+// that fails had queued is over before its code is returned.
+template <typename Fn> static int guarded(Fn fn, EngineBase *eng = nullptr)
 {
   DeviceRestore restore;
   try {
-    fn();
+    try {
+      fn();
+    } catch (...) {
+      if (eng) eng->settle();
+      throw;
+    }
     return AWSEM_OK;
   } catch (CudaError &e) {
     g_last_error = e.what();
@@ -2592,43 +2608,43 @@ int awsem_compute(awsem_system *sys, long long step, const double *x, double *f,
     g_last_error = "awsem_compute: terms must be a non-empty set of AWSEM_TERMS_* bits";
     return AWSEM_EINVAL;
   }
-  return guarded([&] { sys->eng->compute(step, x, f, energies, terms); });
+  return guarded([&] { sys->eng->compute(step, x, f, energies, terms); }, sys->eng.get());
 }
 
 int awsem_replica_set_state(awsem_system *sys, int r, const double *x, const double *v)
 {
   if (!ready(sys)) return AWSEM_EINVAL;
-  return guarded([&] { sys->eng->set_state(r, x, v); });
+  return guarded([&] { sys->eng->set_state(r, x, v); }, sys->eng.get());
 }
 
 int awsem_replica_get_state(awsem_system *sys, int r, double *x, double *v)
 {
   if (!ready(sys)) return AWSEM_EINVAL;
-  return guarded([&] { sys->eng->get_state(r, x, v); });
+  return guarded([&] { sys->eng->get_state(r, x, v); }, sys->eng.get());
 }
 
 int awsem_batch_set_state(awsem_system *sys, const double *x, const double *v)
 {
   if (!ready(sys)) return AWSEM_EINVAL;
-  return guarded([&] { sys->eng->set_state_all(x, v); });
+  return guarded([&] { sys->eng->set_state_all(x, v); }, sys->eng.get());
 }
 
 int awsem_batch_get_state(awsem_system *sys, double *x, double *v)
 {
   if (!ready(sys)) return AWSEM_EINVAL;
-  return guarded([&] { sys->eng->get_state_all(x, v); });
+  return guarded([&] { sys->eng->get_state_all(x, v); }, sys->eng.get());
 }
 
 int awsem_replica_energies(awsem_system *sys, int r, double *energies)
 {
   if (!ready(sys) || !energies) return AWSEM_EINVAL;
-  return guarded([&] { sys->eng->energies(r, energies); });
+  return guarded([&] { sys->eng->energies(r, energies); }, sys->eng.get());
 }
 
 int awsem_replica_forces(awsem_system *sys, int r, double *f)
 {
   if (!ready(sys) || !f) return AWSEM_EINVAL;
-  return guarded([&] { sys->eng->forces(r, f); });
+  return guarded([&] { sys->eng->forces(r, f); }, sys->eng.get());
 }
 
 int awsem_set_state(awsem_system *sys, const double *x, const double *v) { return awsem_replica_set_state(sys, 0, x, v); }
@@ -2651,7 +2667,7 @@ int awsem_run_window(awsem_system *sys, long long nsteps, const awsem_run_params
     g_last_error = "awsem_run_window: a serving handle advances with awsem_server_advance";
     return AWSEM_EINVAL;
   }
-  return guarded([&] { sys->eng->run_window(nsteps, *rp, window_begin, window_end, cont != 0, thermo); });
+  return guarded([&] { sys->eng->run_window(nsteps, *rp, window_begin, window_end, cont != 0, thermo); }, sys->eng.get());
 }
 
 int awsem_run(awsem_system *sys, long long nsteps, const awsem_run_params *rp, double *thermo)
@@ -2668,7 +2684,7 @@ int awsem_run(awsem_system *sys, long long nsteps, const awsem_run_params *rp, d
     g_last_error = "awsem_run: a serving handle advances with awsem_server_advance";
     return AWSEM_EINVAL;
   }
-  return guarded([&] { sys->eng->run(nsteps, *rp, thermo); });
+  return guarded([&] { sys->eng->run(nsteps, *rp, thermo); }, sys->eng.get());
 }
 
 // --------------------------------------------------------------------------
@@ -2724,7 +2740,7 @@ int awsem_server_admit(awsem_system *sys, const awsem_replica_desc *d, long long
     ReplicaArrays ra{d->n_res, d->n_chains, d->chain_len, d->seq, d->ssweight, d->x, d->v, d->n_mem,
                      d->mem_pos, d->mem_len, d->mem_weight, d->mem_seq, d->mem_ca, d->mem_cb};
     got = sys->eng->admit(ra, d->seed, nsteps, t_start, t_stop);
-  });
+  }, sys->eng.get());
   if (rc != AWSEM_OK) return rc;
   if (got < 0) {
     g_last_error = "awsem_server_admit: no free slot, residue range or memory-record room now";
@@ -2770,7 +2786,7 @@ int awsem_server_admit_prepared(awsem_system *sys, awsem_request *req, long long
   int rc = guarded([&] {
     CK(cudaSetDevice(sys->eng->device));
     got = sys->eng->admit_prepared(req->prep, req->seed, nsteps, t_start, t_stop);
-  });
+  }, sys->eng.get());
   if (rc != AWSEM_OK) return rc;
   if (got < 0) {
     g_last_error = "awsem_server_admit_prepared: no free slot, residue range or memory-record room now";
@@ -2793,7 +2809,7 @@ int awsem_server_advance(awsem_system *sys, long long nsteps)
   return guarded([&] {
     CK(cudaSetDevice(sys->eng->device));
     sys->eng->advance(nsteps);
-  });
+  }, sys->eng.get());
 }
 
 int awsem_server_progress(awsem_system *sys, int slot, long long *done, long long *total)
@@ -2813,7 +2829,7 @@ int awsem_server_collect(awsem_system *sys, int slot, double *x, double *v, doub
     if (x || v) sys->eng->get_state(slot, x, v);
     if (energies) sys->eng->energies(slot, energies);
     sys->eng->release(slot);
-  });
+  }, sys->eng.get());
 }
 
 int awsem_server_usage(awsem_system *sys, long long *info)
@@ -2833,7 +2849,7 @@ int awsem_debug_selections(awsem_system *sys, long long step, const double *x, u
 {
   if (!ready(sys) || !x || (cap > 0 && !keys) || !count) return AWSEM_EINVAL;
   long long got = 0;
-  int rc = guarded([&] { got = sys->eng->debug_selections(step, x, keys, cap); });
+  int rc = guarded([&] { got = sys->eng->debug_selections(step, x, keys, cap); }, sys->eng.get());
   *count = got;
   if (rc == AWSEM_OK && got > cap) {
     g_last_error = "selection records exceed the capacity given (" + std::to_string(cap) + " < " +
@@ -2856,7 +2872,7 @@ const char *awsem_kernel_name(int k) { return (k >= 0 && k < AWSEM_NKERNELS) ? k
 int awsem_profile_step(awsem_system *sys, int reps, double *ms)
 {
   if (!ready(sys) || !ms) return AWSEM_EINVAL;
-  return guarded([&] { sys->eng->profile(reps, ms); });
+  return guarded([&] { sys->eng->profile(reps, ms); }, sys->eng.get());
 }
 
 int awsem_autotune(awsem_system *sys, int reps, int *chosen)
@@ -2865,7 +2881,7 @@ int awsem_autotune(awsem_system *sys, int reps, int *chosen)
   return guarded([&] {
     CK(cudaSetDevice(sys->eng->device));
     sys->eng->autotune(reps, chosen);
-  });
+  }, sys->eng.get());
 }
 
 int awsem_set_step_form(awsem_system *sys, int form, int blocks, int stream_warps)

@@ -31,13 +31,17 @@ int last_error = kOk;
 long long pending = 0, captures = 0, live_graphs = 0, live_execs = 0, instantiated = 0, waits = 0;
 bool capture_failed = false;
 std::set<Stream *> streams;
-std::map<std::string, int> fail_after;  // calls of that name in a recording that still succeed
+struct Fail {
+  int after;       // calls of that name that still succeed
+  bool recording;  // of those in a recording, or of all
+};
+std::map<std::string, Fail> fail_after;
 
 // whether this call, part of a recording or not, is the one to fail
 bool fails(const char *name, bool recording)
 {
   auto it = fail_after.find(name);
-  if (it == fail_after.end() || !recording || it->second-- > 0) return false;
+  if (it == fail_after.end() || (it->second.recording && !recording) || it->second.after-- > 0) return false;
   fail_after.erase(it);
   return true;
 }
@@ -65,8 +69,8 @@ int queue(const char *name, void *s)
 
 extern "C" {
 
-// what the tests read and set: from now on, the call of that name after `after` more of them in recordings fails, once
-void fake_fail(const char *name, int after) { fail_after[name] = after; }
+// what the tests read and set: after `after` more calls of that name (in recordings, or all), one fails
+void fake_fail(const char *name, int after, int recording) { fail_after[name] = Fail{after, recording != 0}; }
 int fake_failed(const char *name) { return !fail_after.count(name); }
 long long fake_pending() { return pending; }
 long long fake_capturing()

@@ -60,7 +60,7 @@ x = s.get_state(0)[0]
 one = (lambda: s.compute(x)) if what == "compute" else (lambda: s.run(30))
 for after in range({{b"cudaMemcpyAsync": 2, b"cudaGraphInstantiate": 1}}.get(call, 3)):
     s.set_launch_shapes((1, 148, 148, 0))  # drops what is recorded
-    fake.fake_fail(call, after)
+    fake.fake_fail(call, after, 1)
     for k in range(100):
         no = refused(one)
         assert fake.fake_capturing() == 0 and fake.fake_graphs() == 0, (after, k)
@@ -69,4 +69,35 @@ for after in range({{b"cudaMemcpyAsync": 2, b"cudaGraphInstantiate": 1}}.get(cal
     assert fake.fake_failed(call), after
     assert no == (what == "run"), after
     assert not refused(one), after
+""")
+
+
+@pytest.mark.parametrize("what", ["compute", "run", "set_state", "get_state", "energies", "forces", "serve"])
+def test_failed_call_is_over_when_it_returns(what, host):
+    """A copy that fails in the middle of a call: nothing of the call is still
+    queued on the handle's buffers when it returns, and the next call works."""
+    host(f"""
+what = {what!r}
+if what == "serve":
+    s = engine.AwsemServer(ff, 256, 4, 1 << 16)
+    def one():
+        slot = s.admit(chain(20), 3)
+        s.advance(4)
+        s.collect(slot)
+else:
+    s = system()
+    x, v = s.get_state(0)
+    s.compute(x)
+    one = dict(compute=lambda: s.compute(x), run=lambda: s.run(2), set_state=lambda: s.set_state(x, v),
+               get_state=lambda: s.get_state(0), energies=lambda: s.energies(0), forces=lambda: s.forces(0))[what]
+hit = 0
+for after in range(3 if what == "serve" else 8):
+    fake.fake_fail(b"cudaMemcpyAsync", after, 0)
+    no = refused(one)
+    assert no == bool(fake.fake_failed(b"cudaMemcpyAsync")), after
+    hit += no
+    assert fake.fake_pending() == 0, after
+    fake.fake_fail(b"cudaMemcpyAsync", 10 ** 6, 0)
+    assert not refused(one), after
+assert hit
 """)
