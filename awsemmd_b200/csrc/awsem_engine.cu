@@ -2318,6 +2318,8 @@ template <typename R> class Engine : public EngineBase {
     sl = Slot();
     set_nl_field(&dev::NLState::r_list, 0.f);
     update_launch_extent();
+    // before the caller goes on: awsem_fragmem_noalloc reads the tables on a stream of its own
+    CK(cudaStreamSynchronize(s0));
   }
 
   void usage(long long *info) override

@@ -101,3 +101,16 @@ for after in range(3 if what == "serve" else 8):
     assert not refused(one), after
 assert hit
 """)
+
+
+def test_collected_request_has_left_the_device(host):
+    """The residues and memory tables of a collected request are cleared when
+    the call returns: other entry points read them on other streams."""
+    host("""
+s = engine.AwsemServer(ff, 256, 4, 1 << 16)
+slots = [s.admit(chain(20, k), 3) for k in range(3)]
+s.advance(4)
+for slot in slots:
+    s.collect(slot)
+    assert fake.fake_pending() == 0
+""")
