@@ -843,12 +843,19 @@ template <typename R> class Engine : public EngineBase {
 
   // An evaluation is a fixed sequence on fixed buffers -- positions from the
   // page-locked staging, forces, energies and the list state back to it -- so
-  // that a handle's third call with the same term groups records it in a graph
-  // and later calls launch that (one launch instead of some twenty; the first
-  // two, for programs that need a single evaluation, do not pay for the
-  // recording).  The host waits once, at the end.
-  cudaGraphExec_t eval_graph = nullptr;
-  int eval_groups = -1, eval_calls = 0;
+  // that it is recorded in a graph and later calls launch that, one launch
+  // instead of some twenty.  A graph for each set of term groups, recorded at
+  // the handle's eighth call with them: a recording takes the time of eight
+  // calls' savings (100 residues: 108 us a call queued, 72 recorded, 290 to
+  // record; 2,000: 130, 94 and 370), so programs that need a few evaluations
+  // or ask for different terms in turn do not pay for what they do not use.
+  // The host waits once, at the end.
+  static constexpr int kEvalRecord = 8;
+  struct EvalGraph {
+    cudaGraphExec_t exec = nullptr;
+    int calls = 0;
+  };
+  EvalGraph evals[(dev::G_FIX | dev::G_PAIR | dev::G_BOND) + 1];
 
   // h_io: positions, step counter; then forces, energies, list state
   DBuf<double> results;  // the same on the device
@@ -889,21 +896,17 @@ template <typename R> class Engine : public EngineBase {
       set_list_flags(next_compute_built, 1);
       next_compute_built = 1;
     }
-    if (groups != eval_groups) {
-      release_eval_graph();
-      eval_groups = groups;
-    }
-    eval_calls++;
-    if (eval_calls >= 3 && !eval_graph && !sel_cap) {
+    EvalGraph &eval = evals[groups];
+    if (++eval.calls >= kEvalRecord && !eval.exec && !sel_cap) {
       try {
-        record(eval_graph, [&] { queue_evaluation(groups); });
+        record(eval.exec, [&] { queue_evaluation(groups); });
       } catch (const CudaError &) {
-        eval_calls = 0;  // e.g. no memory for the graph: this call and the next two are queued directly
+        eval.calls = 0;  // e.g. no memory for the graph: this call and the next ones are queued
       }
     }
     for (int attempt = 0; attempt < 2; attempt++) {
-      if (eval_graph && !sel_cap)
-        CK(cudaGraphLaunch(eval_graph, s0));
+      if (eval.exec && !sel_cap)
+        CK(cudaGraphLaunch(eval.exec, s0));
       else
         queue_evaluation(groups);
       CK(cudaGetLastError());
@@ -919,13 +922,6 @@ template <typename R> class Engine : public EngineBase {
     const double *f = h_io.at<double>(io_in());
     for (int k = 0; k < 3 * na; k++) f_ext[k] += f[k];
     if (energies_out) finish_energies(f + 3 * na, energies_out, false);
-  }
-
-  void release_eval_graph()
-  {
-    if (eval_graph) cudaGraphExecDestroy(eval_graph);
-    eval_graph = nullptr;
-    eval_calls = 0;
   }
 
   void finish_energies(const double *e, double *out, bool with_ke)
@@ -1321,7 +1317,10 @@ template <typename R> class Engine : public EngineBase {
 
   void release_graphs()
   {
-    release_eval_graph();
+    for (EvalGraph &e : evals) {
+      if (e.exec) cudaGraphExecDestroy(e.exec);
+      e = EvalGraph();
+    }
     for (auto &row : graphs)
       for (auto &g : row)
         if (g) {

@@ -114,3 +114,26 @@ for slot in slots:
     s.collect(slot)
     assert fake.fake_pending() == 0
 """)
+
+
+@pytest.mark.parametrize("pattern", [[7], [7, 1], [7, 7, 7, 1], [1, 1, 1, 2, 2, 2], [1, 2, 3, 4, 5, 6, 7]])
+def test_force_calls_record_once(pattern, host):
+    """A few force calls record nothing; many record one graph for each set of
+    terms, in whatever turn a host asks for them, until the handle drops them."""
+    host(f"""
+pattern = {pattern!r}
+s = system()
+x = s.get_state(0)[0]
+for t in set(pattern):
+    for k in range(5):
+        s.compute(x, terms=t)
+assert fake.fake_instantiated() == 0
+for k in range(60):
+    for t in pattern:
+        s.compute(x, terms=t)
+assert fake.fake_instantiated() == fake.fake_execs() == len(set(pattern))
+s.set_launch_shapes((1, 148, 148, 0))
+assert fake.fake_execs() == 0
+s.compute(x, terms=pattern[0])
+assert fake.fake_execs() == 0
+""")
