@@ -49,3 +49,24 @@ def test_pair_list_overflow(tmp_path, gpu_lib):
         for k in range(RECORDED):
             _equal(s.compute(x0), want)
         _equal(s.compute(squeezed), tight)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_short_windows(prec, tmp_path, gpu_lib):
+    """A run in windows of seven steps, single steps at first and graphs of
+    five later, has the bits of the run in one call."""
+    from awsemmd_b200 import engine, synth
+
+    c = synth.chain_arrays(35, 6600, n_mem_per_window=2)
+    ff = synth.forcefield_dir(str(tmp_path / "ff"))
+    kw = dict(t_start=330.0, t_stop=290.0, seed=5)
+    n, part = 490, 7
+    with engine.AwsemBatch.from_arrays(ff, [c], precision=prec) as s:
+        s.run_window(n, (0, n), False, **kw)
+        want = (*s.get_state(0), s.forces(0), s.energies(0))
+    with engine.AwsemBatch.from_arrays(ff, [c], precision=prec) as s:
+        for at in range(0, n, part):
+            s.run_window(part, (0, n), at > 0, **kw)
+        got = (*s.get_state(0), s.forces(0), s.energies(0))
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)

@@ -137,3 +137,24 @@ assert fake.fake_execs() == 0
 s.compute(x, terms=pattern[0])
 assert fake.fake_execs() == 0
 """)
+
+
+def test_runs_record_what_they_use(host):
+    """A first short run records single steps only, a long one those and the
+    graph of 25; short windows again and again get the graph of five."""
+    host("""
+with system() as s:
+    s.run(20)
+    assert fake.fake_instantiated() == 1
+    for k in range(10):
+        s.run(19)
+    assert fake.fake_instantiated() == 1
+    for k in range(20):
+        s.run(19)
+    assert fake.fake_instantiated() == 2
+    s.run(30, thermo=True)
+    assert fake.fake_instantiated() == 4
+    s.set_launch_shapes((1, 148, 148, 0))
+    s.run(20)
+    assert fake.fake_execs() == 1
+""")
