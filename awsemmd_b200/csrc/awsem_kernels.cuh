@@ -40,6 +40,7 @@
 #include "awsem_device.cuh"
 #include "awsem_fragmem.cuh"
 #include "awsem_gpu.h"
+#include "awsem_grid.h"
 
 namespace awsem {
 namespace dev {
@@ -513,11 +514,6 @@ struct GridArgs {
   int *sorted;          // [n_res] residues of each gridded replica, by cell, at the replica's residue range
 };
 
-__device__ __forceinline__ int grid_coord(float p, float o, float inv, int n)
-{
-  return min(n - 1, max(0, (int) ((p - o) * inv)));
-}
-
 // One block of 1,024 threads per gridded replica, on the steps that rebuild:
 // bounding box and grid shape, each residue's cell and the cell counts, cell
 // starts (exclusive scan, offset by the replica's first residue; a run of
@@ -561,16 +557,9 @@ template <typename R> __global__ void __launch_bounds__(kGridThreads) k_grid_bui
       }
     // cells at least the list radius (plus rounding room) wide
     float cell = a.nl->r_list * 1.0001f + 1e-3f;
+    const float lo3[3] = {sl[0][0], sl[1][0], sl[2][0]}, hi3[3] = {sh[0][0], sh[1][0], sh[2][0]};
     int n[3];
-    for (int it = 0; it < 64; it++) {
-      long long tot = 1;
-      for (int k = 0; k < 3; k++) {
-        n[k] = max(1, (int) ((sh[k][0] - sl[k][0]) / cell) + 1);
-        tot *= n[k];
-      }
-      if (tot <= d.cap) break;
-      cell *= 1.26f;
-    }
+    grid_shape(lo3, hi3, d.cap, cell, n);
     d.ox = sl[0][0];
     d.oy = sl[1][0];
     d.oz = sl[2][0];
@@ -693,13 +682,15 @@ template <typename R> __device__ __forceinline__ void nl_build_one(const StepArg
     a.ncount[i] = count;
     a.cb_build[i] = make_double4(ci.x, ci.y, ci.z, 0.0);
   }
-  int at = base;
+  // unsigned: the pairs of a system that a residue far out has made one single
+  // neighbourhood may pass 2^31 (the first entries beyond the capacity flag it)
+  unsigned at = base;
   if (count)
     scan([&](int it, int j, bool in) {
       const unsigned m = it < 64 ? __shfl_sync(0xffffffffu, it < 32 ? kept[0] : kept[1], it & 31)
                                  : __ballot_sync(0xffffffffu, close(j, in));
-      const int k = at + __popc(m & ((1u << lane) - 1u));
-      if ((m >> lane & 1u) && k < a.pcap) a.pairs[k] = make_int2(i, j);
+      const unsigned k = at + __popc(m & ((1u << lane) - 1u));
+      if ((m >> lane & 1u) && k < (unsigned) a.pcap) a.pairs[k] = make_int2(i, j);
       at += __popc(m);
     });
 }
