@@ -914,8 +914,9 @@ template <typename R> class Engine : public EngineBase {
       // an evaluation whose pair list overflowed runs again on a grown list
       // (it changes no state, unless LAMMPS's lists are emulated, whose
       // per-step bookkeeping it advances: then the overflow is reported)
-      const int ovf = io_state().overflow;
-      if (!ovf || attempt == 1 || lists_emulated()) break;
+      const dev::NLState now = io_state();
+      const int ovf = now.overflow;
+      if (!ovf || attempt == 1 || now.bad_x || lists_emulated()) break;
       grow_pairs(ovf);
     }
     check_state(io_state());
@@ -966,8 +967,12 @@ template <typename R> class Engine : public EngineBase {
   void check_state(const dev::NLState &st)
   {
     if (st.bad_x) {
-      // positions are inputs: the next call with finite ones is clean
+      // positions are inputs: the next call with finite ones is clean, on a
+      // new pair list (this one may lack the pairs of the residue, whose
+      // displacement since no later check could tell)
       set_nl_field(&dev::NLState::bad_x, 0);
+      set_nl_field(&dev::NLState::overflow, 0);
+      set_nl_field(&dev::NLState::r_list, 0.f);
       throw StateError("non-finite atom coordinates; results of this call are invalid");
     }
     if (st.overflow) {

@@ -414,7 +414,10 @@ __device__ __forceinline__ void nl_decide(NLState *nl, int force, long long *ste
   // CA displacement since then + twice the CA-to-contact-bead offset apart
   if (pair_cut > 0.f) need = fmaxf(need, pair_cut + 2.f * sqrtf(ld2) + 2.f * bCA + 0.01f);
   const float disp = sqrtf(d2max);
-  const bool rb = force || r_list <= 0.f || need + 2.f * disp > r_list || (every > 0 && since + 1 >= every);
+  // A list made while some residue was infinitely far from its beads or from
+  // its last place is not kept: no displacement would ever outgrow it.
+  const bool kept = r_list > 0.f && r_list <= 3e38f && need + 2.f * disp <= r_list;
+  const bool rb = force || !kept || (every > 0 && since + 1 >= every);
   // |b(i) - b'(j)| >= |CA(i) - CA(j)| - reach(b) - reach(b'): two residues
   // whose CAs are farther apart than the largest cutoff + reaches of any
   // interacting bead kinds have no bead pair in excluded-volume range
