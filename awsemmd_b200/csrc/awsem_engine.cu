@@ -1760,7 +1760,7 @@ template <typename R> class Engine : public EngineBase {
           cudaGraphExecDestroy(g);
           g = nullptr;
         }
-    single_steps[0] = single_steps[1] = 0;
+      single_steps[1] = 0;  // ... so the graph of five never pays
     }
     long long total = rows;
     capture_for(total, tv);

@@ -150,10 +150,14 @@ with system() as s:
         s.run(19)
     assert fake.fake_instantiated() == 1
     for k in range(20):
+        s.run(3, thermo=True)  # its graphs are made anew for every run
         s.run(19)
-    assert fake.fake_instantiated() == 2
+    assert fake.fake_instantiated() == 2 + 20
     s.run(30, thermo=True)
-    assert fake.fake_instantiated() == 4
+    assert fake.fake_instantiated() == 2 + 20 + 2
+    for k in range(400):
+        s.run(9, thermo=True)
+    assert fake.fake_instantiated() == 2 + 20 + 2 + 400
     s.set_launch_shapes((1, 148, 148, 0))
     s.run(20)
     assert fake.fake_execs() == 1
