@@ -57,8 +57,8 @@ template <typename T> struct DBuf {
   void alloc(size_t count)
   {
     release();
-    n = count;
     if (count) CK(cudaMalloc(&p, count * sizeof(T)));
+    n = count;  // none where there was no memory
   }
   void upload(const std::vector<T> &h, cudaStream_t s)
   {
@@ -657,21 +657,34 @@ template <typename R> class Engine : public EngineBase {
     return c.empty() ? 0 : *std::max_element(c.begin(), c.end());
   }
 
+  // A list that cannot grow, for its indices or for want of memory, keeps its
+  // capacity: the error is this call's, and the next one runs on the old size.
   void resize_pairs(long long newcap)
   {
+    set_nl_field(&dev::NLState::overflow, 0);
+    set_nl_field(&dev::NLState::r_list, 0.f);  // forces a rebuild
     // pair indices (and their complements in the DSSP queue) are ints
     if (newcap >= (1ll << 31)) throw std::invalid_argument("residue pair list exceeds 2^31 pairs");
-    pcap = (int) newcap;
-    pairs.alloc((size_t) pcap);
-    cpairs.alloc((size_t) pcap);
-    seg_n.alloc((size_t) pcap / 32 + 2);
-    hbq.alloc((size_t) 3 * pcap);
-    dev::NLState st;
-    CK(cudaMemcpyAsync(&st, nl.p, sizeof st, cudaMemcpyDeviceToHost, s0));
-    CK(cudaStreamSynchronize(s0));
-    st.overflow = 0;
-    st.r_list = 0.f;  // forces a rebuild
-    CK(cudaMemcpyAsync(nl.p, &st, sizeof st, cudaMemcpyHostToDevice, s0));
+    const int old = pcap;
+    try {
+      alloc_pairs((int) newcap);
+    } catch (const CudaError &) {
+      alloc_pairs(old);
+      throw;
+    }
+  }
+  void alloc_pairs(int cap)
+  {
+    // no list until every part of it is there: the kernels skip what lies past the capacity
+    pcap = 0;
+    for (DBuf<int2> *b : {&pairs, &cpairs}) b->release();
+    seg_n.release();
+    hbq.release();
+    pairs.alloc((size_t) cap);
+    cpairs.alloc((size_t) cap);
+    seg_n.alloc((size_t) cap / 32 + 2);
+    hbq.alloc((size_t) 3 * cap);
+    pcap = cap;
   }
 
   // cell grids of the large replicas (see k_grid_build)

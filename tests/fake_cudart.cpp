@@ -36,6 +36,8 @@ struct Fail {
   bool recording;  // of those in a recording, or of all
 };
 std::map<std::string, Fail> fail_after;
+long long patch_at = -1;  // bytes from the end of the next copy to the host
+int patch_value = 0;
 
 // whether this call, part of a recording or not, is the one to fail
 bool fails(const char *name, bool recording)
@@ -72,6 +74,8 @@ extern "C" {
 // what the tests read and set: after `after` more calls of that name (in recordings, or all), one fails
 void fake_fail(const char *name, int after, int recording) { fail_after[name] = Fail{after, recording != 0}; }
 int fake_failed(const char *name) { return !fail_after.count(name); }
+// an int of the next copy to the host, that far from its end, reads `value`
+void fake_patch(long long from_end, int value) { patch_at = from_end, patch_value = value; }
 long long fake_pending() { return pending; }
 long long fake_capturing()
 {
@@ -102,6 +106,7 @@ int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *,
 
 int cudaMalloc(void **p, size_t n)
 {
+  if (fails("cudaMalloc", false)) return note(kFail);
   return *p = calloc(n ? n : 1, 1), kOk;
 }
 int cudaFree(void *p) { return free(p), kOk; }
@@ -109,10 +114,15 @@ int cudaHostAlloc(void **p, size_t n, unsigned) { return *p = calloc(n ? n : 1, 
 int cudaFreeHost(void *p) { return free(p), kOk; }
 int cudaMemcpy(void *d, const void *s, size_t n, int) { return memmove(d, s, n), kOk; }
 int cudaMemset(void *d, int v, size_t n) { return memset(d, v, n), kOk; }
-int cudaMemcpyAsync(void *d, const void *s, size_t n, int, void *st)
+int cudaMemcpyAsync(void *d, const void *s, size_t n, int kind, void *st)
 {
   const int rc = queue("cudaMemcpyAsync", st);
-  if (!rc && !(st && static_cast<Stream *>(st)->capture)) memmove(d, s, n);
+  if (rc || (st && static_cast<Stream *>(st)->capture)) return rc;
+  memmove(d, s, n);
+  if (kind == 2 && patch_at >= 0 && patch_at <= (long long) n) {  // device to host
+    memcpy(static_cast<char *>(d) + n - patch_at, &patch_value, sizeof patch_value);
+    patch_at = -1;
+  }
   return rc;
 }
 int cudaMemsetAsync(void *d, int v, size_t n, void *st)

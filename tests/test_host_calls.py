@@ -1,13 +1,22 @@
 """The engine's host code on a CUDA runtime without a device
 (fake_cudart.cpp, preloaded into a child process): what its calls queue, record
 and wait for, and what they leave behind when a runtime call fails."""
+import functools
 import os
 import subprocess
 import sys
 
 import pytest
 
+from awsemmd_b200 import build
+
 HERE = os.path.dirname(os.path.abspath(__file__))
+
+OFFSET = """
+#include <cstdio>
+#include "awsem_kernels.cuh"
+int main() { printf("%d", (int) (sizeof(awsem::dev::NLState) - offsetof(awsem::dev::NLState, overflow))); }
+"""
 
 PRELUDE = """
 import ctypes, sys, tempfile
@@ -36,7 +45,16 @@ def host(gpu_lib, tmp_path_factory):
     lib = str(d / "fake_cudart.so")
     subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-o", lib, os.path.join(HERE, "fake_cudart.cpp")], check=True)
 
+    @functools.cache
+    def overflow():
+        (d / "o.cu").write_text(OFFSET)
+        inc = ["-I" + os.path.join(os.path.dirname(HERE), p) for p in ("awsemmd_b200/csrc", "include")]
+        subprocess.run([build.nvcc(), "-std=c++17", "--expt-relaxed-constexpr", *build.ARCH, *inc, "-o", str(d / "o"), str(d / "o.cu")],
+                       check=True)
+        return subprocess.run([str(d / "o")], check=True, capture_output=True, text=True).stdout
+
     def run(script):
+        script = script.replace("OVERFLOW_FROM_END", overflow()) if "OVERFLOW_FROM_END" in script else script
         code = PRELUDE.format(root=os.path.dirname(HERE), lib=lib, tmp=str(d)) + script
         r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, LD_PRELOAD=lib), capture_output=True, text=True,
                            timeout=300)
@@ -161,4 +179,26 @@ with system() as s:
     s.set_launch_shapes((1, 148, 148, 0))
     s.run(20)
     assert fake.fake_execs() == 1
+""")
+
+
+@pytest.mark.parametrize("after", range(4))
+def test_pair_list_that_cannot_grow(after, host):
+    """No memory for a larger pair list: the call that needed it fails, the
+    handle keeps the list it had."""
+    host(f"""
+s = system()
+x = s.get_state(0)[0]
+s.compute(x)
+capacity = s.model_info()[5]
+assert capacity > 0
+fake.fake_patch(OVERFLOW_FROM_END, 10 ** 6)  # the evaluation reports an overflow
+fake.fake_fail(b"cudaMalloc", {after}, 0)
+assert refused(lambda: s.compute(x))
+assert fake.fake_failed(b"cudaMalloc")
+assert s.model_info()[5] == capacity
+assert not refused(lambda: s.compute(x))
+fake.fake_patch(OVERFLOW_FROM_END, 10 ** 6)
+s.compute(x)
+assert s.model_info()[5] == 2 * 10 ** 6
 """)
