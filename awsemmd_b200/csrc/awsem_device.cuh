@@ -24,6 +24,7 @@ namespace dev {
 
 constexpr double F_SCALE = 4294967296.0;        // forces: 2^32
 constexpr double F_UNSCALE = 1.0 / 4294967296.0;
+constexpr double F_LOW_SCALE = 1048576.0, F_LOW_UNSCALE = 1.0 / 1048576.0;  // parts of a unit of 1 / F_SCALE
 constexpr double D_SCALE = 1099511627776.0;     // densities, xi: 2^40
 constexpr double D_UNSCALE = 1.0 / 1099511627776.0;
 

@@ -229,7 +229,7 @@ template <typename R> class Engine : public EngineBase {
   DBuf<int> zim;                   // membrane zones
   DBuf<int> vfm_start, vfm_j;      // vector fragment memory records
   DBuf<double> vfm_angle;
-  int efix_slots = 5;
+  int efix_slots = 6;
   int fm_groups = 0, fm_dsplit = 1;
   DBuf<double> thermo_rows;
   DBuf<int> res_sys, sys_begin, sys_end;
@@ -548,7 +548,7 @@ template <typename R> class Engine : public EngineBase {
       cr_w.upload(in.cr.w.empty() ? std::vector<double>{0.0} : in.cr.w, s0);
       cr_r0.upload(in.cr.r0.empty() ? std::vector<double>{0.0} : in.cr.r0, s0);
     }
-    efix_slots = (in.ff.p.terms & (T_SSB | T_DH | T_CONTREST)) ? 8 : 5;
+    efix_slots = (in.ff.p.terms & (T_SSB | T_DH | T_CONTREST)) ? 9 : 6;
     if (in.ff.p.terms & T_VFM) {
       std::vector<int> st(in.vfm.start);
       st.resize((size_t) nn + 1, st.empty() ? 0 : st.back());

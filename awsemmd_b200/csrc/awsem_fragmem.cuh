@@ -243,11 +243,26 @@ __device__ __forceinline__ void fm_row_geometry(const Pos &pos, int i, int j, V3
 // rows add their forces on i to memory as they end, from differences formed
 // again there: what the record loop holds then fits 12 warps per
 // multiprocessor without spills (all in registers: 242, 8 warps).
+// Where energies go: per residue (stride 1) or all to one total (stride 0),
+// in fixed point (2^-32), and apart from it what rounding the rows to that
+// left (2^-52), so that an energy is as good as its rows' sums and still the
+// same however the rows are spread over units.  (FP64, nine to fourteen
+// residues: 5e-10 off with rows in 2^-32 alone, below 7e-12 now.)
+struct FMEnergy {
+  unsigned long long *high, *low;
+  int stride;
+};
+__device__ __forceinline__ int fix_low(double v, long long high)
+{
+  return __double2int_rn((v * F_SCALE - (double) high) * F_LOW_SCALE);
+}
+
 template <typename R> struct FMSums {
   R es = 0, fs[4] = {0, 0, 0, 0}, es1 = 0, fs1[4] = {0, 0, 0, 0};  // even and odd records
   R et = 0, ft[4] = {0, 0, 0, 0};                                  // FP64: the row's pieces so far
   long long fca[3] = {0, 0, 0}, fcb[3] = {0, 0, 0};
-  long long e = 0;  // fixed point by row: the same whatever rows share a unit
+  long long e = 0;  // the rows' energies in fixed point, the same whatever rows share a unit ...
+  int e_low = 0;    // ... and what their roundings left
 
   // a piece ends
   __device__ __forceinline__ void end_piece()
@@ -270,7 +285,10 @@ template <typename R> struct FMSums {
   __device__ __forceinline__ void end_row(R scale, R s2, const R r[4], const V3<R> dv[4], const Pos &pos, int ii,
                                           bool live, int j, unsigned long long *facc)
   {
-    e += fix_force((double) (scale * et));
+    const double er = (double) (scale * et);
+    const long long ef = fix_force(er);
+    e += ef;
+    e_low += fix_low(er, ef);
     long long fja[3] = {0, 0, 0}, fjb[3] = {0, 0, 0};
     if constexpr (sizeof(R) == 8) {
       V3<R> dp[4];
@@ -315,21 +333,26 @@ template <typename R> struct FMSums {
     }
   }
   // the unit ends
-  __device__ __forceinline__ void end_unit(bool live, int i, unsigned long long *facc, unsigned long long *e_acc,
-                                           int e_stride)
+  __device__ __forceinline__ void end_unit(bool live, int i, unsigned long long *facc, const FMEnergy &to)
   {
     if (sizeof(R) == 4 && live) {
       red_add3(facc + (size_t) 9 * i, fca);
       red_add3(facc + (size_t) 9 * i + 3, fcb);
     }
     long long en = live ? e : 0;
-    if (e_stride) {
-      if (en) atomicAdd(e_acc + (size_t) i * e_stride, (unsigned long long) en);
-    } else {
+    int lo = live ? e_low : 0;
+    size_t at = i;
+    if (to.stride == 0) {  // one total: the warp's first
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) en += __shfl_xor_sync(0xffffffffu, en, o);
-      if ((threadIdx.x & 31) == 0 && en) atomicAdd(e_acc, (unsigned long long) en);
+      for (int o = 16; o > 0; o >>= 1) {
+        en += __shfl_xor_sync(0xffffffffu, en, o);
+        lo += __shfl_xor_sync(0xffffffffu, lo, o);
+      }
+      if ((threadIdx.x & 31) != 0) en = lo = 0;
+      at = 0;
     }
+    if (en) atomicAdd(to.high + at, (unsigned long long) en);
+    if (lo) atomicAdd(to.low + at, (unsigned long long) (long long) lo);
   }
 };
 
@@ -361,13 +384,12 @@ __device__ __forceinline__ bool fm_join_pieces(FMSums<float> &) { return true; }
 // Work unit w of the fragment-memory term, records loaded into registers.  `pos(r, b)` returns the FP64
 // position of residue r's CA (b = 0) or CB (b = 1); forces go to `facc`
 // ([atom][3], atom = 3 r + b, fixed point).  Energies are added in fixed
-// point to e_acc[i * e_stride] (per residue with e_stride = 1; one total
-// with e_stride = 0).  sig[s] is the Gaussian variance of sequence
+// point to `en`.  sig[s] is the Gaussian variance of sequence
 // separation s, |s|^(2 * sigma_exp) (fix_backbone.cpp:4126).
 template <bool COEF, typename R, class Pos>
 __device__ __forceinline__ void fragmem_unit_reg_t(int w, const FMSlices<R> &t, const double *sig, int n,
                                                    const Pos &pos, unsigned long long *facc,
-                                                   unsigned long long *e_acc, int e_stride)
+                                                   const FMEnergy &en)
 {
   const int lane = threadIdx.x & 31;
   const FMUnit u = fm_unit(w, t);
@@ -405,17 +427,17 @@ __device__ __forceinline__ void fragmem_unit_reg_t(int w, const FMSlices<R> &t, 
     if (sizeof(R) == 8 && t.psplit > 1 && !fm_join_pieces(sum)) return;
     sum.end_row(scale, s2, r, dv, pos, ii, live, j, facc);
   }
-  sum.end_unit(live, i, facc, e_acc, e_stride);
+  sum.end_unit(live, i, facc, en);
 }
 
 template <typename R, class Pos>
 __device__ __forceinline__ void fragmem_unit_reg(int w, const FMSlices<R> &t, const double *sig, int n, const Pos &pos,
-                                                 unsigned long long *facc, unsigned long long *e_acc, int e_stride)
+                                                 unsigned long long *facc, const FMEnergy &en)
 {
   if (t.coef)
-    fragmem_unit_reg_t<true>(w, t, sig, n, pos, facc, e_acc, e_stride);
+    fragmem_unit_reg_t<true>(w, t, sig, n, pos, facc, en);
   else
-    fragmem_unit_reg_t<false>(w, t, sig, n, pos, facc, e_acc, e_stride);
+    fragmem_unit_reg_t<false>(w, t, sig, n, pos, facc, en);
 }
 
 // FP32 rows by two warps: warp h (0, 1) of the pair takes a row's even or odd
@@ -428,8 +450,7 @@ __device__ __forceinline__ void fragmem_unit_reg(int w, const FMSlices<R> &t, co
 // series, four loads in flight, held the call at 36 us.
 template <bool COEF, class Pos>
 __device__ __forceinline__ void fragmem_unit_pair(int w, int h, const FMSlices<float> &t, const double *sig, int n,
-                                                  const Pos &pos, unsigned long long *facc, unsigned long long *e_acc,
-                                                  int e_stride, float *xch, int bar)
+                                                  const Pos &pos, unsigned long long *facc, const FMEnergy &en, float *xch, int bar)
 {
   constexpr int kAhead = 8;
   const int lane = threadIdx.x & 31;
@@ -486,7 +507,7 @@ __device__ __forceinline__ void fragmem_unit_pair(int w, int h, const FMSlices<f
       for (int k = 0; k < 4; k++) sum.fs[k] = 0.f;
     }
   }
-  if (!h) sum.end_unit(live, i, facc, e_acc, e_stride);
+  if (!h) sum.end_unit(live, i, facc, en);
 }
 
 // A launch with one warp (FP64; a block where it shares a row) or one
@@ -494,7 +515,7 @@ __device__ __forceinline__ void fragmem_unit_pair(int w, int h, const FMSlices<f
 template <typename R> constexpr int kFmUnitWarps = sizeof(R) == 4 ? 2 : 1;
 template <typename R, class Pos>
 __device__ __forceinline__ void fragmem_warp(const FMSlices<R> &t, const double *sig, int n, const Pos &pos,
-                                             unsigned long long *facc, unsigned long long *e_acc, int e_stride)
+                                             unsigned long long *facc, const FMEnergy &en)
 {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if constexpr (sizeof(R) == 4) {
@@ -502,12 +523,12 @@ __device__ __forceinline__ void fragmem_warp(const FMSlices<R> &t, const double 
     const int pair = (threadIdx.x >> 6) & 1;
     if (w / 2 >= t.groups * t.dsplit) return;  // both warps of the pair
     if (t.coef)
-      fragmem_unit_pair<true>(w / 2, w & 1, t, sig, n, pos, facc, e_acc, e_stride, xch[pair], 1 + pair);
+      fragmem_unit_pair<true>(w / 2, w & 1, t, sig, n, pos, facc, en, xch[pair], 1 + pair);
     else
-      fragmem_unit_pair<false>(w / 2, w & 1, t, sig, n, pos, facc, e_acc, e_stride, xch[pair], 1 + pair);
+      fragmem_unit_pair<false>(w / 2, w & 1, t, sig, n, pos, facc, en, xch[pair], 1 + pair);
   } else {
     const int u = t.psplit > 1 ? (int) blockIdx.x : w;
-    if (u < t.groups * t.dsplit) fragmem_unit_reg(u, t, sig, n, pos, facc, e_acc, e_stride);
+    if (u < t.groups * t.dsplit) fragmem_unit_reg(u, t, sig, n, pos, facc, en);
   }
 }
 
@@ -594,7 +615,7 @@ __device__ __forceinline__ void load_record_shared(const double *rf, int rec, do
 template <bool COEF, typename R, class Pos>
 __device__ __forceinline__ bool fragmem_unit_bulk_t(int w, const FMSlices<R> &t, const double *sig, int n,
                                                     const Pos &pos, unsigned long long *facc,
-                                                    unsigned long long *e_acc, int e_stride, int *timed_out,
+                                                    const FMEnergy &en, int *timed_out,
                                                     unsigned char *wsm, unsigned &kbase)
 {
   const int lane = threadIdx.x & 31;
@@ -705,18 +726,18 @@ __device__ __forceinline__ bool fragmem_unit_bulk_t(int w, const FMSlices<R> &t,
   sum.end_piece();
   if (sizeof(R) == 8 && t.psplit > 1 && !fm_join_pieces(sum)) return true;
   sum.end_row(scale, s2, r, dv, pos, ii, live, j, facc);
-  sum.end_unit(live, i, facc, e_acc, e_stride);
+  sum.end_unit(live, i, facc, en);
   return true;
 }
 
 template <typename R, class Pos>
 __device__ __forceinline__ bool fragmem_unit_bulk(int w, const FMSlices<R> &t, const double *sig, int n,
                                                   const Pos &pos, unsigned long long *facc,
-                                                  unsigned long long *e_acc, int e_stride, int *timed_out,
+                                                  const FMEnergy &en, int *timed_out,
                                                   unsigned char *wsm, unsigned &kbase)
 {
-  return t.coef ? fragmem_unit_bulk_t<true>(w, t, sig, n, pos, facc, e_acc, e_stride, timed_out, wsm, kbase)
-                : fragmem_unit_bulk_t<false>(w, t, sig, n, pos, facc, e_acc, e_stride, timed_out, wsm, kbase);
+  return t.coef ? fragmem_unit_bulk_t<true>(w, t, sig, n, pos, facc, en, timed_out, wsm, kbase)
+                : fragmem_unit_bulk_t<false>(w, t, sig, n, pos, facc, en, timed_out, wsm, kbase);
 }
 
 // A warp's copy ring: its stage mbarriers, initialised once (the phase
@@ -737,8 +758,7 @@ __device__ __forceinline__ void fragmem_ring_init(unsigned char *wsm)
 // units, and the launch ends within one unit of balance.
 template <typename R, class Pos>
 __device__ __forceinline__ void fragmem_warp_take(const FMSlices<R> &t, const double *sig, int n, const Pos &pos,
-                                                  unsigned long long *facc, unsigned long long *e_acc,
-                                                  int e_stride, int *timed_out, unsigned char *wsm, int *next)
+                                                  unsigned long long *facc, const FMEnergy &en, int *timed_out, unsigned char *wsm, int *next)
 {
   const int units = t.groups * t.dsplit, lane = threadIdx.x & 31;
   fragmem_ring_init(wsm);
@@ -750,7 +770,7 @@ __device__ __forceinline__ void fragmem_warp_take(const FMSlices<R> &t, const do
       __syncthreads();
       const int u = s_u;
       if (u >= units) return;
-      const bool ok = fragmem_unit_bulk(u, t, sig, n, pos, facc, e_acc, e_stride, timed_out, wsm, kbase);
+      const bool ok = fragmem_unit_bulk(u, t, sig, n, pos, facc, en, timed_out, wsm, kbase);
       if (!__syncthreads_and(ok)) return;
     }
   }
@@ -759,7 +779,7 @@ __device__ __forceinline__ void fragmem_warp_take(const FMSlices<R> &t, const do
     if (lane == 0) u = atomicAdd(next, 1);
     u = __shfl_sync(0xffffffffu, u, 0);
     if (u >= units) return;
-    if (!fragmem_unit_bulk(u, t, sig, n, pos, facc, e_acc, e_stride, timed_out, wsm, kbase)) return;
+    if (!fragmem_unit_bulk(u, t, sig, n, pos, facc, en, timed_out, wsm, kbase)) return;
   }
 }
 

@@ -156,7 +156,8 @@ template <typename R> struct StepArgs {
   int *hbq;
   // energies summed over pairs, in 2^-32 fixed point (sums independent of
   // order): [0] DSSP, [1] P_AP, [2] fragment memory, [3] water, [4] excluded
-  // volume between residues; [5][n_res]
+  // volume between residues, [5] what rounding left of the fragment-memory
+  // rows (FMEnergy), then the pair terms of pair_extra_pass; [slots][n_res]
   long long *e_fix;
   // density sums in 2^-40 fixed point: [0] water, [1] helix, [2] raw xi_water; [3][n_res]
   long long *dacc;
@@ -186,7 +187,7 @@ template <typename R> struct StepArgs {
   const double *charge;          // [n]: charge of the residue
   const int *cr_start, *cr_j;    // contact restraints of residue i (i < j): [cr_start[i], cr_start[i+1])
   const double *cr_w, *cr_r0;
-  int efix_slots;                // fixed-point energy slots in use (5, or 8 with the pair terms above)
+  int efix_slots;                // fixed-point energy slots in use (6, or 9 with the pair terms above)
   const int *zim;                // [n]: membrane zone (1, 2, 3) of the residue
   const int *vfm_start, *vfm_j;  // vector fragment memory records of residue i (i < j)
   const double *vfm_angle;
@@ -201,6 +202,12 @@ template <typename R> struct StepArgs {
   unsigned long long *sel, *sel_n;
   long long sel_cap;
 };
+
+template <typename R> __device__ __forceinline__ FMEnergy fm_energy(const StepArgs<R> &a)
+{
+  unsigned long long *e = (unsigned long long *) a.e_fix;
+  return {e + (size_t) 2 * a.s.n_res, e + (size_t) 5 * a.s.n_res, 1};
+}
 
 enum Group { G_FIX = 1, G_PAIR = 2, G_BOND = 4 };
 
@@ -1587,9 +1594,7 @@ template <typename R> __global__ void __launch_bounds__(128, kFmMinBlocks<R>) k_
   extern __shared__ __align__(128) unsigned char fm_smem[];
   const BeadPos<R> pos{&a.s};
   unsigned char *wsm = fm_smem + (threadIdx.x >> 5) * fm_warp_smem<R>(a.fm.coef != nullptr);
-  fragmem_warp_take(a.fm, p.fm_sigma_sq, a.s.n_res, pos, a.s.facc,
-                    (unsigned long long *) (a.e_fix + (size_t) 2 * a.s.n_res), 1, &a.nl->fm_timeout, wsm,
-                    &a.nl->fm_next);
+  fragmem_warp_take(a.fm, p.fm_sigma_sq, a.s.n_res, pos, a.s.facc, fm_energy(a), &a.nl->fm_timeout, wsm, &a.nl->fm_next);
 }
 
 // Table fragment memory of residue i and separation slot jo
@@ -1703,16 +1708,16 @@ template <typename R> __global__ void k_list_hold(StepArgs<R> a)
 //     (:8112-8113, :6307-6363), evaluated for every CA pair of the fix's half
 //     list -- CAs within the pair-list cutoff plus the skin at the replica's
 //     last list build, 1-2 bonded pairs removed -- on the contact beads.
-// Forces to the fixed-point accumulators; energies to fixed-point slots 5-7.
+// Forces to the fixed-point accumulators; energies to fixed-point slots 6-8.
 template <typename R> __device__ __forceinline__ void pair_extra_pass(const StepArgs<R> &a, const FFParams &p, Span sp)
 {
   const DevSys<R> &s = a.s;
   const int n = s.n_res;
   if (!(a.groups & G_FIX)) return;
   const uint32_t T = p.terms;
-  unsigned long long *e_ssb = (unsigned long long *) a.e_fix + (size_t) 5 * n;
-  unsigned long long *e_dh = (unsigned long long *) a.e_fix + (size_t) 6 * n;
-  unsigned long long *e_cr = (unsigned long long *) a.e_fix + (size_t) 7 * n;
+  unsigned long long *e_ssb = (unsigned long long *) a.e_fix + (size_t) 6 * n;
+  unsigned long long *e_dh = (unsigned long long *) a.e_fix + (size_t) 7 * n;
+  unsigned long long *e_cr = (unsigned long long *) a.e_fix + (size_t) 8 * n;
   const double cut = p.pair_list_cutoff + a.nl->lst_skin, cutsq = cut * cut;
   const int np = min(a.nl->npairs, a.pcap);
   for (int q = sp.t; q < np; q += sp.nthr) {
@@ -2243,8 +2248,8 @@ __global__ void k_thermo(const double *e_res, const long long *e_fix, int efix_s
     double fx = 0.0;
     for (int t = 1; t < E_FIX_TERMS; t++) fx += e_res[(size_t) t * n_res + r];
     long long fq = e_fix[r] + e_fix[(size_t) n_res + r] + e_fix[(size_t) 2 * n_res + r] + e_fix[(size_t) 3 * n_res + r];
-    for (int k = 5; k < efix_slots; k++) fq += e_fix[(size_t) k * n_res + r];
-    fx += (double) fq * F_UNSCALE;
+    for (int k = 6; k < efix_slots; k++) fq += e_fix[(size_t) k * n_res + r];
+    fx += ((double) fq + (double) e_fix[(size_t) 5 * n_res + r] * F_LOW_UNSCALE) * F_UNSCALE;
     acc[0] += fx;
     acc[1] += e_res[(size_t) E_PAIR * n_res + r] + (double) e_fix[(size_t) 4 * n_res + r] * F_UNSCALE;
     acc[2] += e_res[(size_t) E_BOND * n_res + r];
@@ -2326,11 +2331,13 @@ __device__ __forceinline__ double energy_slot(const double *e_res, const long lo
   double acc = 0.0;
   // pair-summed energies are kept in fixed point (e_fix slots)
   int k = t == E_DSSP ? 0 : t == E_PAP ? 1 : t == E_FRAGMEM ? 2 : t == E_WATER ? 3 : t == E_PAIR ? 4
-              : t == E_SSB ? 5 : t == E_DH ? 6 : t == E_CONT_REST ? 7 : -1;
+              : t == E_SSB ? 6 : t == E_DH ? 7 : t == E_CONT_REST ? 8 : -1;
   if (k >= efix_slots) k = -1;
   const long long *fx = k >= 0 ? e_fix + (size_t) k * n_res : nullptr;
+  const long long *low = t == E_FRAGMEM ? e_fix + (size_t) 5 * n_res : nullptr;
   for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x)
-    acc += e_res[(size_t) t * n_res + r] + (fx ? (double) fx[r] * F_UNSCALE : 0.0);
+    acc += e_res[(size_t) t * n_res + r] +
+           (fx ? ((double) fx[r] + (low ? (double) low[r] * F_LOW_UNSCALE : 0.0)) * F_UNSCALE : 0.0);
   sh[threadIdx.x] = acc;
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {

@@ -27,8 +27,8 @@
 namespace awsem {
 namespace noalloc {
 
-// fixed-point (2^-32) force accumulator [atoms][3], then one slot for the
-// fixed-point energy (padded to keep the array a multiple of 256 bytes)
+// fixed-point (2^-32) force accumulator [atoms][3], then two slots for the
+// energy's parts (padded to keep the array a multiple of 256 bytes)
 constexpr int kEnergySlot = AWSEM_NOALLOC_MAX_ATOMS * 3;
 static __device__ __align__(256) unsigned long long g_facc[AWSEM_NOALLOC_MAX_ATOMS * 3 + 32];
 
@@ -84,7 +84,7 @@ __global__ void k_clear(unsigned long long *facc, int n)
 {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) facc[k] = 0ull;
-  if (k == 0) facc[kEnergySlot] = 0ull;
+  if (k == 0) facc[kEnergySlot] = facc[kEnergySlot + 1] = 0ull;
 }
 
 struct SigmaTable {
@@ -108,14 +108,16 @@ __global__ void __launch_bounds__(128) k_fragmem(const double *x, int n_res, dev
                                                  unsigned long long *facc)
 {
   const CallerPos pos{x};
-  dev::fragmem_warp(t, sig.v, n_res, pos, facc, facc + kEnergySlot, 0);
+  dev::fragmem_warp(t, sig.v, n_res, pos, facc, dev::FMEnergy{facc + kEnergySlot, facc + kEnergySlot + 1, 0});
 }
 
 __global__ void k_unfix(const unsigned long long *facc, int n, double *f, double *energy)
 {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) f[k] = (double) (long long) facc[k] * dev::F_UNSCALE;
-  if (k == 0) *energy = (double) (long long) facc[kEnergySlot] * dev::F_UNSCALE;
+  if (k == 0)
+    *energy = ((double) (long long) facc[kEnergySlot] + (double) (long long) facc[kEnergySlot + 1] * dev::F_LOW_UNSCALE) *
+              dev::F_UNSCALE;
 }
 
 template <typename R> dev::FMSlices<R> slices(const FMView &v)

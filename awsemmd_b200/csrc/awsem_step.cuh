@@ -144,7 +144,7 @@ __device__ __forceinline__ void fragmem_take_units(const StepArgs<R> &a, const F
                                                    bool ring, unsigned char *wsm, unsigned &kbase)
 {
   const BeadPos<R> pos{&a.s};
-  unsigned long long *e_acc = (unsigned long long *) (a.e_fix + (size_t) 2 * a.s.n_res);
+  const FMEnergy en = fm_energy(a);
   const int lane = threadIdx.x & 31;
   while (true) {
     int u = 0;
@@ -152,11 +152,11 @@ __device__ __forceinline__ void fragmem_take_units(const StepArgs<R> &a, const F
     u = __shfl_sync(0xffffffffu, u, 0);
     if (u >= q.fm_units) return;
     if (ring) {
-      if (!fragmem_unit_bulk(u, a.fm, p.fm_sigma_sq, a.s.n_res, pos, a.s.facc, e_acc, 1, &a.nl->fm_timeout, wsm,
+      if (!fragmem_unit_bulk(u, a.fm, p.fm_sigma_sq, a.s.n_res, pos, a.s.facc, en, &a.nl->fm_timeout, wsm,
                              kbase))
         return;
     } else {
-      fragmem_unit_reg(u, a.fm, p.fm_sigma_sq, a.s.n_res, pos, a.s.facc, e_acc, 1);
+      fragmem_unit_reg(u, a.fm, p.fm_sigma_sq, a.s.n_res, pos, a.s.facc, en);
     }
   }
 }
