@@ -1574,7 +1574,7 @@ template <typename R> class Engine : public EngineBase {
     v.min_sep = in.ff.p.fm_min_sep;
     v.groups = fm_groups;
     v.dsplit = fm_dsplit;
-    v.psplit = fm_psplit(fm_groups);
+    v.psplit = sizeof(R) == 4 ? fm_pair() : fm_psplit(fm_groups);
     v.n_res = n();
     v.is_double = sizeof(R) == sizeof(double);
     v.sigma_sq = in.ff.p.fm_sigma_sq;
@@ -1635,6 +1635,14 @@ template <typename R> class Engine : public EngineBase {
   {
     if (sizeof(R) == 4 || server || fm_dsplit != in.ff.p.fm_nd || fm_rowmax > dev::kFmPiece * dev::kFmBlockPieces) return 1;
     return groups * fm_dsplit <= 4 * sms_ ? dev::kFmBlockPieces : 1;
+  }
+  // FP32 units of the allocation-free call: warp pairs, unless a unit is a few records (8,000 residues, us: 18 records
+  // a unit 24 by a warp and 25.5 by a pair, 48 26.3 and 25.9, 120 35 and 29; several separations a unit, 36 records,
+  // 28.3 and 27.9)
+  int fm_pair() const
+  {
+    const int nd = std::max(in.ff.p.fm_nd, 1);
+    return server || fm_rowmax * ((nd + fm_dsplit - 1) / fm_dsplit) >= 36 ? 2 : 1;
   }
   int fm_units() const { return std::min(fm_groups, (n_run() + 31) / 32) * fm_dsplit; }
 

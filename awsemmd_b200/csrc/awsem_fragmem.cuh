@@ -50,7 +50,8 @@ template <typename R> struct FMSlices {
   int groups;       // G = ceil(n_res / 32)
   int dsplit;       // separation chunks per group (warps per group)
   int psplit;       // warps per unit: 4 (FP64, one separation a chunk, rows of at most 4 pieces: a block
-                    // takes a unit, a warp each piece of its row) or 1
+                    // takes a unit, a warp each piece of its row), 2 (FP32 without a copy ring: a warp
+                    // each set of sums) or 1
   long long wait_limit;  // SM clock cycles a warp waits for one stage's copies before it gives up
   unsigned hold_tx;      // bytes each stage expects beyond its copies: 0, or (tests of the give-up
                          // path) 16, which never arrive, so every stage wait runs out
@@ -510,15 +511,18 @@ __device__ __forceinline__ void fragmem_unit_pair(int w, int h, const FMSlices<f
   if (!h) sum.end_unit(live, i, facc, en);
 }
 
-// A launch with one warp (FP64; a block where it shares a row) or one
-// warp pair (FP32) per work unit, 128 threads a block
-template <typename R> constexpr int kFmUnitWarps = sizeof(R) == 4 ? 2 : 1;
+// A launch with one warp per work unit, 128 threads a block; where psplit says
+// so, a block (FP64, sharing a row) or a warp pair (FP32)
 template <typename R, class Pos>
 __device__ __forceinline__ void fragmem_warp(const FMSlices<R> &t, const double *sig, int n, const Pos &pos,
                                              unsigned long long *facc, const FMEnergy &en)
 {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if constexpr (sizeof(R) == 4) {
+    if (t.psplit == 1) {
+      if (w < t.groups * t.dsplit) fragmem_unit_reg(w, t, sig, n, pos, facc, en);
+      return;
+    }
     __shared__ float xch[2][320];
     const int pair = (threadIdx.x >> 6) & 1;
     if (w / 2 >= t.groups * t.dsplit) return;  // both warps of the pair

@@ -155,8 +155,7 @@ void fragmem_noalloc(int device, const FMView &v, const double *d_x, double *d_f
   int n3 = 3 * n_atoms, tb = 256;
   k_clear<<<(n3 + tb - 1) / tb, tb, 0, stream>>>(facc, n3);
   if (v.nd > 0) {
-    const int warps = v.is_double ? dev::kFmUnitWarps<double> : dev::kFmUnitWarps<float>;
-    int blocks = (v.groups * v.dsplit * v.psplit * warps * 32 + 127) / 128;
+    const int blocks = (v.groups * v.dsplit * v.psplit * 32 + 127) / 128;
     if (v.is_double)
       k_fragmem<double><<<blocks, 128, 0, stream>>>(d_x, v.n_res, slices<double>(v), sig, facc);
     else
