@@ -36,6 +36,7 @@
 #pragma once
 
 #include "awsem_device.cuh"
+#include "awsem_gauss.h"
 
 namespace awsem {
 namespace dev {
@@ -87,57 +88,41 @@ __device__ __forceinline__ float fm_gauss(float x)
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// FP64 Gaussians: e^x for x <= 0 by the table method of P. T. P. Tang ("Table-
-// driven implementation of the exponential function in IEEE floating-point
-// arithmetic", ACM TOMS 15 (1989)) in units of ln2 / 32: z = 32 x / ln2 = 32 m
-// + j + f with |f| <= 1/2, e^x = 2^m 2^(j/32) (1 + p(f)), p the Taylor
-// polynomial of 2^(f/32) - 1 to f^6 (remainder below 4e-18).  The row's factor
-// carries the 32 / ln2, so z - (32 m + j) is exact.  Lane j of the warp holds
-// 2^(j/32), read by a shuffle.  No branches and no calls: the exponentials of
-// a record pair are formed side by side.  Arguments below -708 (the padding's
-// -1e59 among them) give 0.  Every lane of the warp takes part.
-__device__ const double kExp2Of32nds[32] = {
-    0x1.0000000000000p+0, 0x1.059b0d3158574p+0, 0x1.0b5586cf9890fp+0, 0x1.11301d0125b51p+0,
-    0x1.172b83c7d517bp+0, 0x1.1d4873168b9aap+0, 0x1.2387a6e756238p+0, 0x1.29e9df51fdee1p+0,
-    0x1.306fe0a31b715p+0, 0x1.371a7373aa9cbp+0, 0x1.3dea64c123422p+0, 0x1.44e086061892dp+0,
-    0x1.4bfdad5362a27p+0, 0x1.5342b569d4f82p+0, 0x1.5ab07dd485429p+0, 0x1.6247eb03a5585p+0,
-    0x1.6a09e667f3bcdp+0, 0x1.71f75e8ec5f74p+0, 0x1.7a11473eb0187p+0, 0x1.82589994cce13p+0,
-    0x1.8ace5422aa0dbp+0, 0x1.93737b0cdc5e5p+0, 0x1.9c49182a3f090p+0, 0x1.a5503b23e255dp+0,
-    0x1.ae89f995ad3adp+0, 0x1.b7f76f2fb5e47p+0, 0x1.c199bdd85529cp+0, 0x1.cb720dcef9069p+0,
-    0x1.d5818dcfba487p+0, 0x1.dfc97337b9b5fp+0, 0x1.ea4afa2a490dap+0, 0x1.f50765b6e4540p+0,
-};
+// FP64 Gaussians (awsem_gauss.h).  Lane j of the warp holds 2^(j/32), read by
+// shuffles.  No branches and no calls: the exponentials of a record pair are
+// formed side by side.  Every lane of the warp takes part.
+__device__ const double kExp2Of32nds[32] = {AWSEM_EXP2_OF_32NDS};
+__device__ const unsigned kExp2Of32ndsLow[32] = {AWSEM_EXP2_OF_32NDS_LOW};
 template <typename R> struct GaussTable {};
 template <> struct GaussTable<double> {
   double t = kExp2Of32nds[threadIdx.x & 31];
+  unsigned low = kExp2Of32ndsLow[threadIdx.x & 31];
 };
 template <int N> __device__ __forceinline__ void fm_gauss(const double (&z)[N], const GaussTable<double> &tab, double (&g)[N])
 {
-  const double magic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low word is the nearest integer
+  constexpr double poly[5] = {AWSEM_GAUSS_POLY};
   double y[N], f[N], q[N];
 #pragma unroll
-  for (int k = 0; k < N; k++) y[k] = __dadd_rn(z[k], magic);
+  for (int k = 0; k < N; k++) y[k] = __dadd_rn(z[k], kGaussRound);
 #pragma unroll
-  for (int k = 0; k < N; k++) f[k] = __dsub_rn(z[k], __dsub_rn(y[k], magic));
+  for (int k = 0; k < N; k++) f[k] = __dsub_rn(z[k], __dsub_rn(y[k], kGaussRound)), q[k] = kGaussTop;
 #pragma unroll
-  for (int k = 0; k < N; k++) q[k] = __fma_rn(f[k], 0x1.430912f86c787p-43, 0x1.5d87fe78a6731p-35);
+  for (int c = 0; c < 5; c++)
 #pragma unroll
-  for (int k = 0; k < N; k++) q[k] = __fma_rn(f[k], q[k], 0x1.3b2ab6fba4e77p-27);
+    for (int k = 0; k < N; k++) q[k] = __fma_rn(f[k], q[k], poly[c]);
 #pragma unroll
-  for (int k = 0; k < N; k++) q[k] = __fma_rn(f[k], q[k], 0x1.c6b08d704a0c0p-20);
-#pragma unroll
-  for (int k = 0; k < N; k++) q[k] = __fma_rn(f[k], q[k], 0x1.ebfbdff82c58fp-13);
-#pragma unroll
-  for (int k = 0; k < N; k++) q[k] = __dmul_rn(f[k], __fma_rn(f[k], q[k], 0x1.62e42fefa39efp-6));
+  for (int k = 0; k < N; k++)
+    q[k] = __fma_rn(f[k], q[k], __hiloint2double((int) __shfl_sync(0xffffffffu, tab.low, __double2loint(y[k]) & 31), 0));
 #pragma unroll
   for (int k = 0; k < N; k++) {
     const int n = __double2loint(y[k]);
     const double t = __shfl_sync(0xffffffffu, tab.t, n & 31);
     const double s = __hiloint2double(__double2hiint(t) + ((n >> 5) << 20), __double2loint(t));
-    g[k] = z[k] < -708.0 * 0x1.71547652b82fep+5 ? 0.0 : __fma_rn(s, q[k], s);
+    g[k] = z[k] < kGaussLeast ? 0.0 : __fma_rn(s, q[k], s);
   }
 }
 __device__ __forceinline__ float fm_k2(float s2) { return -1.4426950408889634f / (2.f * s2); }
-__device__ __forceinline__ double fm_k2(double s2) { return -0x1.71547652b82fep+5 / (2.0 * s2); }  // 32 / ln2
+__device__ __forceinline__ double fm_k2(double s2) { return gauss_factor(s2); }
 
 // One record's four Gaussians g_k (times the record's coefficient when the
 // coefficients are not uniform): es += sum g_k, fs_k += g_k dr_k.  The row's
