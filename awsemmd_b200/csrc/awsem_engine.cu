@@ -16,6 +16,7 @@
 #include "awsem_gpu.h"
 #include "awsem_step.cuh"
 #include "awsem_model.h"
+#include "awsem_shape.h"
 
 namespace awsem {
 
@@ -395,7 +396,10 @@ template <typename R> class Engine : public EngineBase {
   // list, beside the density pass; above, the near list that pass writes.  A
   // third of the listed pairs are out of reach, but on 2,000 residues the
   // detection and hydrogen-bond passes are on the critical path (39 -> 36 us
-  // a step), on 40,000 218 against 223; on 283,000 1,182 against 1,041.
+  // a step).  The whole list against the near one, mixed form: 43,000 residues
+  // 167 against 171, 65,000 226 and 231, 87,000 301 and 288, 131,000 441 and
+  // 411.  (FP64, whose fragment memory leaves more room, would gain by the
+  // whole list further up: 131,000 706 and 717.)
   static constexpr int kPairWhole = 65536;
 
   // selection records of one evaluation (awsem_debug_selections)
@@ -1651,19 +1655,12 @@ template <typename R> class Engine : public EngineBase {
   int fm_grid = 0;
   bool shapes_given = false;  // by the caller or the autotuner: kept
 
-  // Default shapes for `groups` residue groups.  Separations split over enough
-  // warps to fill the multiprocessors, over two at least (units that end
-  // closer together: 1,024 chains 881 -> 860 us a step); FP64 rows are units
-  // of their own at every size.  FP32 units are taken by three blocks a
-  // multiprocessor: HBM is saturated (0.31 ms against 0.34 with a warp a unit
-  // on 1,858 MB) and the pair passes beside it find room (1,024 chains 925 ->
-  // 867 us a step, 40,000 residues 173 -> 171; two blocks 934 and 165).
   void fm_default_shape(int groups)
   {
     if (shapes_given) return;
-    const int nd = std::max(in.ff.p.fm_nd, 1), g = std::max(groups, 1);
-    fm_dsplit = sizeof(R) == 8 ? nd : std::max(std::min(2, nd), std::min(nd, (16 * sms_ + g - 1) / g));
-    fm_grid = sizeof(R) == 8 ? 0 : 3 * sms_;
+    const FMShape shape = fm_shape(sizeof(R) == 8, groups, in.ff.p.fm_nd, sms_);
+    fm_dsplit = shape.dsplit;
+    fm_grid = shape.grid;
   }
   int fm_blocks() const
   {
