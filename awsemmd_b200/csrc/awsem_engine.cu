@@ -1528,10 +1528,10 @@ template <typename R> class Engine : public EngineBase {
     bool fm = p.fm_nd > 0;
     for (int r = 0; r < reps; r++) {
       for (int k = 0; k < AWSEM_NKERNELS; k++) {
+        if (k == K_NL_DECIDE) continue;  // by the last block of k_prepare
         CK(cudaEventRecord(ev[2 * k], s0));
         switch (k) {
           case K_PREPARE: dev::k_prepare<R><<<nb, tb, 0, s0>>>(a, p, 0, dstep.p); break;
-          case K_NL_DECIDE: break;  // taken by the last block of k_prepare
           case K_NL_BUILD: launch_list_build(a, s0); break;
           case K_DENSITY: dev::k_density<R><<<pair_blocks, tb, 0, s0>>>(a, p); break;
           case K_RESIDUE: launch_residue(a, s0); break;
@@ -1553,6 +1553,7 @@ template <typename R> class Engine : public EngineBase {
       }
       CK(cudaStreamSynchronize(s0));
       for (int k = 0; k < AWSEM_NKERNELS; k++) {
+        if (k == K_NL_DECIDE) continue;
         float t = 0.f;
         CK(cudaEventElapsedTime(&t, ev[2 * k], ev[2 * k + 1]));
         acc[k] += t;

@@ -192,7 +192,7 @@ template <typename R> struct StepArgs {
   const int *vfm_start, *vfm_j;  // vector fragment memory records of residue i (i < j)
   const double *vfm_angle;
   int groups;       // AWSEM_TERMS_* bits: 1 fix backbone, 2 pair vexcluded, 4 bonds
-  long long *step;   // device step counter (advanced by k_nl_decide)
+  long long *step;   // device step counter (advanced by the list decision)
   // replicas: residue -> replica, replica residue ranges, Langevin seeds
   // (res_sys < 0: residue of no replica, skipped)
   const int *res_sys, *sys_begin, *sys_end;
@@ -2321,9 +2321,7 @@ __global__ void k_q_sum(const double *partial, int n, double qnorm, double *out)
   if (threadIdx.x == 0) *out = sh[0] * qnorm;
 }
 
-// Per-term sums of each replica's residues in a fixed tree order
-// (block (t, r) sums energy slot t of replica rep0 + r)
-// energy slot t summed over residues [r0, r1) in a fixed tree order (a block of 256 threads; thread 0 has the sum)
+// Energy slot t summed over residues [r0, r1) in a fixed tree order (a block of 256 threads; thread 0 has the sum)
 __device__ __forceinline__ double energy_slot(const double *e_res, const long long *e_fix, int efix_slots, int n_res, int t,
                                               int r0, int r1)
 {
@@ -2347,6 +2345,7 @@ __device__ __forceinline__ double energy_slot(const double *e_res, const long lo
   return sh[0];
 }
 
+// Per-term sums of each replica's residues: block (t, r) sums energy slot t of replica rep0 + r
 __global__ void k_energy_reduce(const double *e_res, const long long *e_fix, int efix_slots, int n_res,
                                 const int *sys_begin, const int *sys_end, double *out, int rep0)
 {

@@ -284,7 +284,9 @@ int awsem_neighbor_stats(awsem_system *sys, int *nbuilds, double *radius, int *m
 /* Current MD step counter. */
 long long awsem_step(const awsem_system *sys);
 
-/* Kernels of one MD step, in launch order (names for awsem_profile_step). */
+/* Kernels of one MD step, in launch order (names for awsem_profile_step).
+ * nl_decide is not a kernel of its own: prepare's last block takes the pair
+ * list's decision, and its time reads 0. */
 #define AWSEM_NKERNELS 12
 const char *awsem_kernel_name(int k);
 
