@@ -171,7 +171,7 @@ class EngineBase {
   virtual PreparedDeleter prepared_deleter() const = 0;
   virtual void progress(int slot, long long *done, long long *total) = 0;
   virtual void advance(long long nsteps) = 0;
-  virtual void release(int slot) = 0;
+  virtual void collect(int slot, double *x_ext, double *v_ext, double *energies) = 0;
   virtual void usage(long long *info) = 0;
 };
 
@@ -1129,12 +1129,24 @@ template <typename R> class Engine : public EngineBase {
       get_atoms(a0, na, from, to);
       return;
     }
-    const std::vector<int> &ext = in.ext_of[rep];
+    queue_replica(rep, from, to);
+    CK(cudaStreamSynchronize(s0));
+    take_replica(rep, to);
+  }
+  // ... in the engine's order to h_io, and from there once that has been waited for
+  void queue_replica(int rep, const double *from[2], double *to[2])
+  {
+    const int a0 = rep_atom0(rep), na = rep_atoms(rep);
     const size_t bytes = sizeof(double) * 3 * na;
     h_io.need(2 * bytes);
     for (int k = 0; k < 2; k++)
       if (to[k] && na) CK(cudaMemcpyAsync(h_io.p + k * bytes, from[k] + 3 * (size_t) a0, bytes, cudaMemcpyDeviceToHost, s0));
-    CK(cudaStreamSynchronize(s0));
+  }
+  void take_replica(int rep, double *to[2]) const
+  {
+    const int na = rep_atoms(rep);
+    const std::vector<int> &ext = in.ext_of[rep];
+    const size_t bytes = sizeof(double) * 3 * na;
     for (int k = 0; k < 2; k++) {
       if (!to[k]) continue;
       const double *h = h_io.at<double>(k * bytes);
@@ -1892,11 +1904,15 @@ template <typename R> class Engine : public EngineBase {
   void energies(int rep, double *out) override
   {
     check_rep(rep);
+    queue_energies(rep);
+    CK(cudaStreamSynchronize(s0));
+    finish_energies(h_call.at<double>(kHostEnergy), out, true);
+  }
+  void queue_energies(int rep)
+  {
     reduce_energies(rep, 1);
     CK(cudaMemcpyAsync(h_call.p + kHostEnergy, energy.p + (size_t) rep * E_SLOTS, sizeof(double) * E_SLOTS,
                        cudaMemcpyDeviceToHost, s0));
-    CK(cudaStreamSynchronize(s0));
-    finish_energies(h_call.at<double>(kHostEnergy), out, true);
   }
 
   void forces(int rep, double *f_ext) override
@@ -2351,26 +2367,35 @@ template <typename R> class Engine : public EngineBase {
     check_state(*h_call.at<dev::NLState>(0));
   }
 
-  void release(int k) override
+  // A finished request's results (each may be null), and its room free again.
+  // One wait for all of it, before the caller goes on: awsem_fragmem_noalloc
+  // reads the tables on a stream of its own.  (A wait for each part: 45 us a
+  // request without the release's, 55 with it, 43 in one.)
+  void collect(int k, double *x_ext, double *v_ext, double *energies_out) override
   {
     check_slot(k);
     Slot &sl = slots[k];
     const int base = sl.base, n = sl.n_res, nd = in.ff.p.fm_nd;
+    const double *from[2] = {x.p, v.p};
+    double *to[2] = {x_ext, v_ext};
+    if (x_ext || v_ext) queue_replica(k, from, to);
+    if (energies_out) queue_energies(k);
+    set_nl_field(&dev::NLState::r_list, 0.f);
     // its residues back to residues of no request, its window and range to none
     dev::k_release<<<(n + 127) / 128, 128, 0, s0>>>(
         dev::ReleaseArgs{res_sys.p, res_flags.p, res_chain.p, bond_i.p, fm_slen.p, fm_soff.p, excl_self.p, excl_next.p, x.p,
                          v.p, sys_begin.p, sys_end.p, slot_run.p, base, n, k, nd > 0 ? base / 32 * nd : 0,
                          nd > 0 ? sl.groups * nd : 0});
     CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(s0));
+    take_replica(k, to);
+    if (energies_out) finish_energies(h_call.at<double>(kHostEnergy), energies_out, true);
     give_range(free_groups, base / 32, sl.groups);
     give_range(free_stripes, sl.stripe0, sl.stripes);
     in.sys_res_begin[k] = in.sys_res_end[k] = 0;
     in.ext_of[k].clear();
     sl = Slot();
-    set_nl_field(&dev::NLState::r_list, 0.f);
     update_launch_extent();
-    // before the caller goes on: awsem_fragmem_noalloc reads the tables on a stream of its own
-    CK(cudaStreamSynchronize(s0));
   }
 
   void usage(long long *info) override
@@ -2879,9 +2904,7 @@ int awsem_server_collect(awsem_system *sys, int slot, double *x, double *v, doub
     long long done = 0, total = 0;
     sys->eng->progress(slot, &done, &total);
     if (done < total) throw std::invalid_argument("awsem_server_collect: the request has not finished");
-    if (x || v) sys->eng->get_state(slot, x, v);
-    if (energies) sys->eng->energies(slot, energies);
-    sys->eng->release(slot);
+    sys->eng->collect(slot, x, v, energies);
   }, sys->eng.get());
 }
 

@@ -134,6 +134,32 @@ for slot in slots:
 """)
 
 
+def test_request_is_collected_whole(host):
+    """A collection waits once; one that fails before it has cleared the
+    request leaves it to be collected again."""
+    host("""
+s = engine.AwsemServer(ff, 256, 4, 1 << 16)
+for call in (b"", b"cudaMemcpyAsync", b"cudaLaunchKernel"):
+    for after in range(4):
+        slot = s.admit(chain(20, after), 3)
+        s.advance(4)
+        natoms = dict(s.natoms)
+        if call:
+            fake.fake_fail(call, after, 0)
+        waits = fake.fake_waits()
+        no = refused(lambda: s.collect(slot))
+        if no:
+            s.natoms = natoms
+            assert s.usage()["requests"] == 1
+            fake.fake_fail(call, 10 ** 6, 0)
+            waits = fake.fake_waits()
+            s.collect(slot)
+        assert no == (bool(call) and after < {b"cudaMemcpyAsync": 4, b"cudaLaunchKernel": 2}[call]), (call, after)
+        assert fake.fake_waits() == waits + 1 and fake.fake_pending() == 0
+        assert s.usage()["requests"] == 0
+""")
+
+
 @pytest.mark.parametrize("pattern", [[7], [7, 1], [7, 7, 7, 1], [1, 1, 1, 2, 2, 2], [1, 2, 3, 4, 5, 6, 7]])
 def test_force_calls_record_once(pattern, host):
     """A few force calls record nothing; many record one graph for each set of
