@@ -496,18 +496,15 @@ __device__ __forceinline__ void fragmem_unit_pair(int w, int h, const FMSlices<f
   if (!h) sum.end_unit(live, i, facc, en);
 }
 
-// A launch with one warp per work unit, 128 threads a block; where psplit says
-// so, a block (FP64, sharing a row) or a warp pair (FP32)
-template <typename R, class Pos>
+// A launch with one warp per work unit, 128 threads a block; a block where
+// psplit says so (FP64, sharing a row), a warp pair with PAIR (FP32: kernels of
+// their own, in one the pair form was 5% slower)
+template <bool PAIR, typename R, class Pos>
 __device__ __forceinline__ void fragmem_warp(const FMSlices<R> &t, const double *sig, int n, const Pos &pos,
                                              unsigned long long *facc, const FMEnergy &en)
 {
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if constexpr (sizeof(R) == 4) {
-    if (t.psplit == 1) {
-      if (w < t.groups * t.dsplit) fragmem_unit_reg(w, t, sig, n, pos, facc, en);
-      return;
-    }
+  if constexpr (PAIR) {
     __shared__ float xch[2][320];
     const int pair = (threadIdx.x >> 6) & 1;
     if (w / 2 >= t.groups * t.dsplit) return;  // both warps of the pair

@@ -61,6 +61,7 @@ static CtxGetCurrentFn ctx_get_current()
 // runtime: at the first call on the device, and again whenever the device's
 // context has changed since (after a cudaDeviceReset the old address is
 // gone).
+static void load_kernels();
 static unsigned long long *scratch(int device)
 {
   if (device < 0 || device >= kMaxDevices) throw std::invalid_argument("device index out of range");
@@ -74,6 +75,7 @@ static unsigned long long *scratch(int device)
     void *p = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_facc);
     if (e != cudaSuccess) throw std::runtime_error(std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
+    load_kernels();
     c.addr = (unsigned long long *) p;
     c.ctx = ctx;
   }
@@ -103,12 +105,24 @@ struct CallerPos {
 
 // The engine's fragment-memory warp routine on the caller's positions, so
 // both entry points give the same forces bit for bit.
-template <typename R>
+template <typename R, bool PAIR>
 __global__ void __launch_bounds__(128) k_fragmem(const double *x, int n_res, dev::FMSlices<R> t, SigmaTable sig,
                                                  unsigned long long *facc)
 {
   const CallerPos pos{x};
-  dev::fragmem_warp(t, sig.v, n_res, pos, facc, dev::FMEnergy{facc + kEnergySlot, facc + kEnergySlot + 1, 0});
+  dev::fragmem_warp<PAIR>(t, sig.v, n_res, pos, facc, dev::FMEnergy{facc + kEnergySlot, facc + kEnergySlot + 1, 0});
+}
+
+// Every form of the kernel is loaded with a device's first call, so that a
+// later call with another handle can be captured.
+static void load_kernels()
+{
+  cudaFuncAttributes a;
+  for (const void *k : {(const void *) k_fragmem<double, false>, (const void *) k_fragmem<float, false>,
+                        (const void *) k_fragmem<float, true>}) {
+    cudaError_t e = cudaFuncGetAttributes(&a, k);
+    if (e != cudaSuccess) throw std::runtime_error(std::string("cudaFuncGetAttributes: ") + cudaGetErrorString(e));
+  }
 }
 
 __global__ void k_unfix(const unsigned long long *facc, int n, double *f, double *energy)
@@ -157,9 +171,11 @@ void fragmem_noalloc(int device, const FMView &v, const double *d_x, double *d_f
   if (v.nd > 0) {
     const int blocks = (v.groups * v.dsplit * v.psplit * 32 + 127) / 128;
     if (v.is_double)
-      k_fragmem<double><<<blocks, 128, 0, stream>>>(d_x, v.n_res, slices<double>(v), sig, facc);
+      k_fragmem<double, false><<<blocks, 128, 0, stream>>>(d_x, v.n_res, slices<double>(v), sig, facc);
+    else if (v.psplit == 2)
+      k_fragmem<float, true><<<blocks, 128, 0, stream>>>(d_x, v.n_res, slices<float>(v), sig, facc);
     else
-      k_fragmem<float><<<blocks, 128, 0, stream>>>(d_x, v.n_res, slices<float>(v), sig, facc);
+      k_fragmem<float, false><<<blocks, 128, 0, stream>>>(d_x, v.n_res, slices<float>(v), sig, facc);
   }
   k_unfix<<<(n3 + tb - 1) / tb, tb, 0, stream>>>(facc, n3, d_f, d_energy);
   cudaError_t e = cudaGetLastError();
