@@ -224,11 +224,6 @@ __device__ __forceinline__ void fm_row_geometry(const Pos &pos, int i, int j, V3
   for (int k = 0; k < 4; k++) r[k] = m_sqrt(norm2(dv[k]));
 }
 
-// Sums of the rows of one unit: the running sums of the current piece, in FP64
-// the row's, and in FP32 the unit's forces on residue i in fixed point.  FP64
-// rows add their forces on i to memory as they end, from differences formed
-// again there: what the record loop holds then fits 12 warps per
-// multiprocessor without spills (all in registers: 242, 8 warps).
 // Where energies go: per residue (stride 1) or all to one total (stride 0),
 // in fixed point (2^-32), and apart from it what rounding the rows to that
 // left (2^-52), so that an energy is as good as its rows' sums and still the
@@ -243,6 +238,11 @@ __device__ __forceinline__ int fix_low(double v, long long high)
   return __double2int_rn((v * F_SCALE - (double) high) * F_LOW_SCALE);
 }
 
+// Sums of the rows of one unit: the running sums of the current piece, in FP64
+// the row's, and in FP32 the unit's forces on residue i in fixed point.  FP64
+// rows add their forces on i to memory as they end, from differences formed
+// again there: what the record loop holds then fits 12 warps per
+// multiprocessor without spills (162 registers).
 template <typename R> struct FMSums {
   R es = 0, fs[4] = {0, 0, 0, 0}, es1 = 0, fs1[4] = {0, 0, 0, 0};  // even and odd records
   R et = 0, ft[4] = {0, 0, 0, 0};                                  // FP64: the row's pieces so far

@@ -1585,8 +1585,8 @@ template <typename R> struct BeadPos {
   __device__ __forceinline__ V3<double> operator()(int r, int b) const { return bead(*s, r, b ? B_CB : B_CA); }
 };
 
-// Blocks per multiprocessor it is compiled for.  FP64 (61 chains, alone): 168 registers, three blocks 88 us, where two
-// blocks of 242 took 94 and four of 128 (spilling) 98.
+// Blocks per multiprocessor it is compiled for.  FP64, 61 and 240 chains alone: three blocks (162 registers) 84 and
+// 230 us, two (188) 85 and 256, four (128, spilling) 95 and 272.
 template <typename R> constexpr int kFmMinBlocks = sizeof(R) == 4 ? 4 : 3;
 // 128 threads, fm_warp_smem<R>(coef) bytes of dynamic shared memory per warp
 template <typename R> __global__ void __launch_bounds__(128, kFmMinBlocks<R>) k_fragmem(StepArgs<R> a, FFParams p)
